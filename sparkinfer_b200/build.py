@@ -22,7 +22,7 @@ OUTPUT = PKG / "_b12x_b200.so"
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
-    "-shared", "-Xcompiler", "-fPIC",
+    "-shared", "-Xcompiler", "-fPIC", "--threads", "0",
     "--fmad=false",  # the quantizers must round every product; nothing else is FMA-bound
 ]
 

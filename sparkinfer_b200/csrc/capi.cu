@@ -1,17 +1,7 @@
 // Host side of the C ABI: argument checks, TMA descriptor encoding, tile choice, launches.
-#include "../../include/b12x_b200.h"
-
-#include <cuda.h>
-#include <cuda_runtime.h>
-
-#include <cstdio>
-#include <cstdlib>
-#include <cstring>
-#include <atomic>
-#include <mutex>
+#include "host_common.cuh"
 
 #include "gemm_blockscaled.cuh"
-#include "gemm_block_fp8.cuh"
 #include "gemm_blockscaled_pair.cuh"
 #include "gemm_smallm.cuh"
 #include "quantize.cuh"
@@ -20,220 +10,10 @@
 #include "bmm_mxfp8.cuh"
 
 namespace b12x_b200 {
-namespace {
 
 thread_local char g_last_error[256] = "";
 
-int fail_cuda(cudaError_t err, const char* what) {
-  snprintf(g_last_error, sizeof(g_last_error), "%s: %s", what, cudaGetErrorString(err));
-  return B12X_B200_ERR_CUDA;
-}
-
-int fail(int code, const char* what) {
-  snprintf(g_last_error, sizeof(g_last_error), "%s", what);
-  return code;
-}
-
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// The driver entry point is looked up through the runtime so the library carries no link-time
-// dependency on libcuda (it must load on machines without a driver).
-EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void* sym = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(sym);
-  });
-  return fn;
-}
-
-// Checks of the optional epilogue description that do not depend on the kernel. `allow_quant`:
-// whether the kernel that will run can re-quantize its output (only the decode kernel can).
-int check_epilogue(const b12x_b200_epilogue_t* e, int c_dtype, int64_t n, bool allow_quant) {
-  if (!e) return B12X_B200_OK;
-  if (e->bias) {
-    const uintptr_t align = (c_dtype == B12X_B200_FP32) ? 3 : 1;
-    if (reinterpret_cast<uintptr_t>(e->bias) & align)
-      return fail(B12X_B200_ERR_ALIGNMENT, "bias must be aligned to its element size");
-  }
-  if (e->quant_values) {
-    if (!allow_quant)
-      return fail(B12X_B200_ERR_UNSUPPORTED,
-                  "output re-quantization is available in the decode kernel only (M <= 128)");
-    if (c_dtype == B12X_B200_FP32)
-      return fail(B12X_B200_ERR_UNSUPPORTED, "output re-quantization needs a BF16 or FP16 output");
-    if (n % 32 != 0 || e->quant_cols % 32 != 0 || e->quant_col0 % 32 != 0 || e->quant_col0 < 0 ||
-        e->quant_col0 + n > e->quant_cols || e->quant_ld < e->quant_cols ||
-        e->quant_cols > INT32_MAX)
-      return fail(B12X_B200_ERR_INVALID_ARGUMENT,
-                  "re-quantized output: N, quant_col0 and quant_cols must be multiples of 32, "
-                  "quant_col0 + N <= quant_cols <= quant_ld");
-  } else if (e->quant_scale_rows || e->quant_scale_mma) {
-    return fail(B12X_B200_ERR_INVALID_ARGUMENT, "quant scales given without quant_values");
-  }
-  return B12X_B200_OK;
-}
-
-// K-major byte matrix [rows, row_bytes] -> boxes of 128 bytes x box_rows, 128-byte swizzle.
-int make_operand_map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
-                        uint32_t box_rows) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return fail(B12X_B200_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
-  const cuuint64_t dims[2] = {row_bytes, rows};
-  const cuuint64_t strides[1] = {row_bytes};
-  const cuuint32_t box[2] = {128, box_rows};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  const CUresult r =
-      fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box,
-         elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    snprintf(g_last_error, sizeof(g_last_error), "cuTensorMapEncodeTiled failed (%d)", int(r));
-    return B12X_B200_ERR_CUDA;
-  }
-  return B12X_B200_OK;
-}
-
-// Stack of `groups` K-major byte matrices [groups, rows, row_bytes] -> boxes of 128 bytes x
-// box_rows x 1 group, 128-byte swizzle. A box never crosses into the next group: rows at or
-// beyond `rows` are out of bounds and read as zeros.
-int make_operand_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
-                     uint32_t box_rows, uint64_t groups = 1) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return fail(B12X_B200_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
-  const cuuint64_t dims[3] = {row_bytes, rows, groups};
-  const cuuint64_t strides[2] = {row_bytes, rows * row_bytes};
-  const cuuint32_t box[3] = {128, box_rows, 1};
-  const cuuint32_t elem_strides[3] = {1, 1, 1};
-  const CUresult r =
-      fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box,
-         elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    snprintf(g_last_error, sizeof(g_last_error), "cuTensorMapEncodeTiled failed (%d)", int(r));
-    return B12X_B200_ERR_CUDA;
-  }
-  return B12X_B200_OK;
-}
-
-// Row-major BF16 matrix [rows, cols] with row pitch `ld` elements -> unswizzled boxes of
-// box_cols x box_rows elements (the raw activation rows of the fused-quantizer decode GEMM).
-int make_raw_rows_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
-                      uint32_t box_cols, uint32_t box_rows, uint64_t groups = 1,
-                      uint64_t group_stride = 0) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return fail(B12X_B200_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
-  const cuuint64_t dims[3] = {cols, rows, groups};
-  // Elements between the same row of consecutive groups: group-major [L][rows][ld] by default.
-  const cuuint64_t strides[2] = {ld * 2, (group_stride ? group_stride : rows * ld) * 2};
-  const cuuint32_t box[3] = {box_cols, box_rows, 1};
-  const cuuint32_t elem_strides[3] = {1, 1, 1};
-  const CUresult r =
-      fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box,
-         elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    snprintf(g_last_error, sizeof(g_last_error), "cuTensorMapEncodeTiled(raw rows) failed (%d)", int(r));
-    return B12X_B200_ERR_CUDA;
-  }
-  return B12X_B200_OK;
-}
-
-// Row-major 2-byte matrix [rows, cols] with row pitch `ld` elements -> boxes of 64 columns
-// (128 bytes) x 128 rows, 128-byte swizzle; used for TMA stores of BF16/FP16 outputs.
-int make_output_map_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
-                       uint64_t ld) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return fail(B12X_B200_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
-  const cuuint64_t dims[2] = {cols, rows};
-  const cuuint64_t strides[1] = {ld * 2};
-  const cuuint32_t box[2] = {64, 128};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  const CUresult r =
-      fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base), dims, strides, box,
-         elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-         CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    snprintf(g_last_error, sizeof(g_last_error), "cuTensorMapEncodeTiled(C) failed (%d)", int(r));
-    return B12X_B200_ERR_CUDA;
-  }
-  return B12X_B200_OK;
-}
-
-// The same for a stack of `groups` outputs [groups, rows, ld] (a store never spills into the
-// next group: rows at or beyond `rows` are clipped).
-int make_output_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
-                    uint64_t groups = 1) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return fail(B12X_B200_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
-  const cuuint64_t dims[3] = {cols, rows, groups};
-  const cuuint64_t strides[2] = {ld * 2, rows * ld * 2};
-  const cuuint32_t box[3] = {64, 128, 1};
-  const cuuint32_t elem_strides[3] = {1, 1, 1};
-  const CUresult r =
-      fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box,
-         elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-         CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    snprintf(g_last_error, sizeof(g_last_error), "cuTensorMapEncodeTiled(C) failed (%d)", int(r));
-    return B12X_B200_ERR_CUDA;
-  }
-  return B12X_B200_OK;
-}
-
-struct DeviceInfo {
-  int sm_count = 0;
-  int cc_major = 0;
-};
-
-int device_info(DeviceInfo* out) {
-  static DeviceInfo cache[64];
-  static bool have[64] = {};
-  static std::mutex mu;
-  int dev = 0;
-  cudaError_t err = cudaGetDevice(&dev);
-  if (err != cudaSuccess) return fail_cuda(err, "cudaGetDevice");
-  std::lock_guard<std::mutex> lock(mu);
-  if (dev < 0 || dev >= 64) return fail(B12X_B200_ERR_INVALID_ARGUMENT, "device index out of range");
-  if (!have[dev]) {
-    err = cudaDeviceGetAttribute(&cache[dev].sm_count, cudaDevAttrMultiProcessorCount, dev);
-    if (err != cudaSuccess) return fail_cuda(err, "cudaDeviceGetAttribute");
-    err = cudaDeviceGetAttribute(&cache[dev].cc_major, cudaDevAttrComputeCapabilityMajor, dev);
-    if (err != cudaSuccess) return fail_cuda(err, "cudaDeviceGetAttribute");
-    have[dev] = true;
-  }
-  *out = cache[dev];
-  return B12X_B200_OK;
-}
-
-bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
-
-// Experiment switches, read from the environment once per process (never on the launch path).
-// They exist for measurements of kernel variants; none is part of the interface.
-struct Switches {
-  bool decode_overlap = true;   // programmatic stream serialization for decode GEMMs / quantizers
-  bool pair_tail_split = true;  // split-K the last partial round of the CTA-pair kernel
-  bool bmm_tensor_core = true;  // batched BF16 x MXFP8 product on warp-level MMAs when it fits
-};
-
-const Switches& switches() {
-  static const Switches sw = [] {
-    Switches v;
-    if (const char* e = getenv("B12X_B200_DECODE_OVERLAP")) v.decode_overlap = atoi(e) != 0;
-    if (const char* e = getenv("B12X_B200_PAIR_TAIL_SPLIT")) v.pair_tail_split = atoi(e) != 0;
-    if (const char* e = getenv("B12X_B200_BMM_TENSOR_CORE")) v.bmm_tensor_core = atoi(e) != 0;
-    return v;
-  }();
-  return sw;
-}
+namespace {
 
 // Tile width: fewest (waves x per-tile cost). The per-tile cost model is the bytes one k-step
 // pulls through shared memory, (128 + BN) rows of 128 bytes, which tracks both the MMA time
@@ -330,11 +110,6 @@ int launch_gemm_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const C
                 : launch_gemm_pair_impl<KIND, BN, false>(map_a, map_b, map_c, p, tail, pairs, stream);
 }
 
-// Rows up to which a quantized matrix is taken for an activation (its quantization releases the
-// next kernel early) and a decode GEMM's weight for something a predecessor may just have
-// written (its stream waits for the predecessor). One constant, so the two rules meet.
-constexpr int kEarlyReleaseRows = 128;
-
 // Launch configuration of a row quantizer: 256 threads, programmatic stream serialization.
 struct QuantLaunch {
   cudaLaunchConfig_t cfg;
@@ -363,14 +138,6 @@ int dispatch_block_n(int bn, const CUtensorMap& map_a, const CUtensorMap& map_b,
     default: return fail(B12X_B200_ERR_INVALID_ARGUMENT, "block_n must be 64, 128, 192 or 256");
   }
 }
-
-// Workspace layout shared by the kernels that need scratch (one buffer per stream serves them
-// all, launches on a stream being ordered): 60 KiB of per-tile counters of the decode kernel,
-// 4 KiB of counters of the CTA-pair kernel's split tail, then FP32 partial tiles from 64 KiB on.
-constexpr size_t kSmallMCounterBytes = 60 * 1024;
-constexpr size_t kPairCounterOffset = kSmallMCounterBytes;
-constexpr size_t kPairCounterBytes = 4 * 1024;
-constexpr size_t kWorkspaceHeaderBytes = kPairCounterOffset + kPairCounterBytes;
 
 // Whether (and how) the CTA-pair kernel splits its last, partial round along K: `segments` per
 // leftover tile (0 = no split) and the scratch it needs.
@@ -723,115 +490,6 @@ extern "C" int b12x_b200_quantize_nvfp4_rows(const void* src, int src_dtype, int
                              int(m), int(k), rows_cover, k_cover, k_atoms, early);
   if (err != cudaSuccess) return fail_cuda(err, "quantize_nvfp4_rows launch");
   return B12X_B200_OK;
-}
-
-namespace {
-
-int gemm_block_fp8_impl(const void* a, const float* sfa, const void* b, const float* sfb, void* c,
-                        int c_dtype, const float* alpha, int64_t m, int64_t n, int64_t k,
-                        int64_t ldc, int sm_count, const b12x_b200_epilogue_t* epilogue,
-                        int* status, b12x_b200_stream_t stream) {
-  if (c_dtype < B12X_B200_BF16 || c_dtype > B12X_B200_FP32)
-    return fail(B12X_B200_ERR_INVALID_ARGUMENT, "unknown output dtype");
-  if (m < 0 || n < 0 || k <= 0 || m > INT32_MAX || n > INT32_MAX || k > INT32_MAX)
-    return fail(B12X_B200_ERR_INVALID_ARGUMENT, "bad problem size");
-  if (n % 128 != 0 || k % 128 != 0)
-    return fail(B12X_B200_ERR_UNSUPPORTED, "block-FP8 GEMM needs N and K divisible by 128");
-  if (m == 0 || n == 0) return B12X_B200_OK;
-  if (!a || !b || !sfa || !sfb || !c) return fail(B12X_B200_ERR_INVALID_ARGUMENT, "null pointer");
-  if (ldc < n) return fail(B12X_B200_ERR_INVALID_ARGUMENT, "ldc < n");
-  if (!aligned16(a) || !aligned16(b) || (reinterpret_cast<uintptr_t>(sfa) & 3) ||
-      (reinterpret_cast<uintptr_t>(sfb) & 3))
-    return fail(B12X_B200_ERR_ALIGNMENT, "operands must be 16-byte and scales 4-byte aligned");
-  {
-    const int erc = check_epilogue(epilogue, c_dtype, n, false);
-    if (erc != B12X_B200_OK) return erc;
-  }
-  DeviceInfo info;
-  int rc = device_info(&info);
-  if (rc != B12X_B200_OK) return rc;
-  if (info.cc_major != 10) return fail(B12X_B200_ERR_NO_DEVICE_CODE, "device is not sm_100");
-  const int sms = (sm_count > 0 && sm_count < info.sm_count) ? sm_count : info.sm_count;
-
-  CUtensorMap map_a, map_b;
-  rc = make_operand_map_2d(&map_a, a, uint64_t(m), uint64_t(k), BlockFp8Tile::BM);
-  if (rc != B12X_B200_OK) return rc;
-  rc = make_operand_map_2d(&map_b, b, uint64_t(n), uint64_t(k), BlockFp8Tile::BN);
-  if (rc != B12X_B200_OK) return rc;
-
-  BlockFp8Params p;
-  p.sfa = sfa;
-  p.sfb = sfb;
-  p.c = c;
-  p.alpha = alpha;
-  p.status = status;
-  p.m = int(m);
-  p.n = int(n);
-  p.k = int(k);
-  p.ldc = int(ldc);
-  p.out_dtype = c_dtype;
-  p.tiles_m = int((m + BlockFp8Tile::BM - 1) / BlockFp8Tile::BM);
-  p.tiles_n = int((n + BlockFp8Tile::BN - 1) / BlockFp8Tile::BN);
-  // Tile rows per group of the tile order: 4096 x 18432 x 7168 warm: 4 -> 525, 8 -> 508,
-  // 16 -> 499, 32 (all rows of this problem) -> 496 us.
-  p.group_m = 32;
-  p.bias = epilogue ? epilogue->bias : nullptr;
-  const int64_t tiles = int64_t(p.tiles_m) * p.tiles_n;
-  const int grid = int(tiles < sms ? tiles : sms);
-  static std::atomic<bool> set_for[64];  // zero-initialised; setting the attribute twice is harmless
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !set_for[dev]) {
-    cudaError_t attr_err =
-        cudaFuncSetAttribute(gemm_block_fp8_kernel<false>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, BlockFp8Tile::kSmemBytes);
-    if (attr_err == cudaSuccess)
-      attr_err = cudaFuncSetAttribute(gemm_block_fp8_kernel<true>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      BlockFp8Tile::kSmemBytes);
-    if (attr_err != cudaSuccess) return fail_cuda(attr_err, "cudaFuncSetAttribute");
-    set_for[dev] = true;
-  }
-  // Output through TMA when rows of C are 16-byte aligned 2-byte values; otherwise the
-  // epilogue stores straight from registers.
-  CUtensorMap map_c;
-  memset(&map_c, 0, sizeof(map_c));
-  p.use_tma_store = 0;
-  if (c_dtype != B12X_B200_FP32 && aligned16(c) && (ldc * 2) % 16 == 0) {
-    rc = make_output_map_2d(&map_c, c, uint64_t(m), uint64_t(n), uint64_t(ldc));
-    if (rc != B12X_B200_OK) return rc;
-    p.use_tma_store = 1;
-  }
-  if (p.bias)
-    gemm_block_fp8_kernel<true><<<grid, BlockFp8Tile::kThreads, BlockFp8Tile::kSmemBytes,
-                                  reinterpret_cast<cudaStream_t>(stream)>>>(map_a, map_b, map_c, p);
-  else
-    gemm_block_fp8_kernel<false><<<grid, BlockFp8Tile::kThreads, BlockFp8Tile::kSmemBytes,
-                                   reinterpret_cast<cudaStream_t>(stream)>>>(map_a, map_b, map_c, p);
-  const cudaError_t err = cudaGetLastError();
-  if (err != cudaSuccess) return fail_cuda(err, "gemm_block_fp8 launch");
-  return B12X_B200_OK;
-}
-
-}  // namespace
-
-extern "C" int b12x_b200_gemm_block_fp8(const void* a, const float* sfa, const void* b,
-                                        const float* sfb, void* c, int c_dtype,
-                                        const float* alpha, int64_t m, int64_t n, int64_t k,
-                                        int64_t ldc, int sm_count, int* status,
-                                        b12x_b200_stream_t stream) {
-  return gemm_block_fp8_impl(a, sfa, b, sfb, c, c_dtype, alpha, m, n, k, ldc, sm_count, nullptr,
-                             status, stream);
-}
-
-extern "C" int b12x_b200_gemm_block_fp8_ex(const void* a, const float* sfa, const void* b,
-                                           const float* sfb, void* c, int c_dtype,
-                                           const float* alpha, int64_t m, int64_t n, int64_t k,
-                                           int64_t ldc, int sm_count,
-                                           const b12x_b200_epilogue_t* epilogue, int* status,
-                                           b12x_b200_stream_t stream) {
-  return gemm_block_fp8_impl(a, sfa, b, sfb, c, c_dtype, alpha, m, n, k, ldc, sm_count, epilogue,
-                             status, stream);
 }
 
 namespace {
