@@ -26,7 +26,7 @@ def block_fp8_gemm(a: torch.Tensor, sfa: torch.Tensor, b: torch.Tensor, sfb: tor
     n = b.shape[0]
     want_sfa, want_sfb = (m, k // 128), (n // 128, k // 128)
     if (sf_dtype != "float32" or sf_vec_size != 128 or l != 1 or n % 128 != 0 or k % 128 != 0
-            or tuple(sfa.shape) != want_sfa or tuple(sfb.shape) != want_sfb
+            or sfa.shape != want_sfa or sfb.shape != want_sfb
             or sfa.dtype != torch.float32 or sfb.dtype != torch.float32
             or not sfa.is_contiguous() or not sfb.is_contiguous()):
         raise ValueError(
@@ -40,18 +40,17 @@ def block_fp8_gemm(a: torch.Tensor, sfa: torch.Tensor, b: torch.Tensor, sfb: tor
     for name, t, rows in (("A", a, m), ("B", b, n)):
         if not t.is_cuda:
             raise ValueError(f"{name} must be on CUDA")
-        if t.element_size() != 1 or tuple(t.shape) != (rows, k, 1) or t.stride(1) != 1 \
+        if t.element_size() != 1 or t.shape != (rows, k, 1) or t.stride(1) != 1 \
                 or (rows > 1 and t.stride(0) != k):
             raise ValueError(f"{name} must be a K-major one-byte [{rows}, {k}, 1] tensor")
     if out is None:
         out = torch.empty((m, n, 1), dtype=_C_DTYPES[c_dtype], device=a.device)
-    if tuple(out.shape) != (m, n, 1) or out.dtype != _C_DTYPES[c_dtype] or out.stride(1) != 1:
+    if out.shape != (m, n, 1) or out.dtype != _C_DTYPES[c_dtype] or out.stride(1) != 1:
         raise ValueError(f"out must be {c_dtype} with shape {(m, n, 1)}")
     if alpha is not None and (alpha.dtype != torch.float32 or alpha.numel() != 1):
         raise ValueError("alpha must be a float32 tensor with one element")
     if m == 0:
         return out
-    launch.gemm_block_fp8(a.select(2, 0), sfa, b.select(2, 0), sfb, out.select(2, 0), alpha,
-                          m, n, k, ldc=out.stride(0) if m > 1 else n, sm_count=sm_count,
+    launch.gemm_block_fp8(a, sfa, b, sfb, out, alpha, m, n, k, ldc=out.stride(0) if m > 1 else n, sm_count=sm_count,
                           stream_int=cuda_stream_to_int(stream))
     return out

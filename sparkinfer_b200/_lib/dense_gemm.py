@@ -19,6 +19,7 @@ physical ``[L, M, N]`` storage.
 
 from __future__ import annotations
 
+import functools
 import os
 import logging
 import time
@@ -44,7 +45,15 @@ _ALPHA_ONE_CACHE: dict[tuple[str, int | None], torch.Tensor] = {}
 
 
 def get_num_sm(device: torch.device) -> int:
+    index = getattr(device, "index", None)
+    if index is not None:
+        return _num_sm(index)
     return torch.cuda.get_device_properties(device).multi_processor_count
+
+
+@functools.lru_cache(maxsize=64)
+def _num_sm(index: int) -> int:
+    return torch.cuda.get_device_properties(index).multi_processor_count
 
 
 def _cached_alpha_one(device: torch.device | str) -> torch.Tensor:
@@ -91,10 +100,10 @@ def _check_operand(name: str, t: torch.Tensor, rows: int, row_bytes: int, l: int
         raise ValueError(f"{name} must be on CUDA")
     if t.element_size() != 1:
         raise TypeError(f"{name} must hold one byte per element, got {t.dtype}")
-    if tuple(t.shape) != (rows, row_bytes, l):
+    if t.shape != (rows, row_bytes, l):
         raise ValueError(f"{name} must have shape {(rows, row_bytes, l)}, got {tuple(t.shape)}")
-    want = (row_bytes, 1, rows * row_bytes)
-    if any(t.shape[i] > 1 and t.stride(i) != want[i] for i in range(3)):
+    have, want = t.stride(), (row_bytes, 1, rows * row_bytes)
+    if have != want and any(t.shape[i] > 1 and have[i] != want[i] for i in range(3)):
         raise ValueError(
             f"{name} must be K-major over physical [L, rows, K] storage (strides {want}), "
             f"got {t.stride()}")
@@ -117,9 +126,10 @@ def _dense_gemm_launch_flat(a, b, sfa, sfb, c, alpha, *, n: int, k: int, l: int,
         raise ValueError("SFA must be the (32,4,m_tiles,4,k_tiles,L) view over dense atom storage")
     if not mma_view_is_canonical(sfb, n, k, sf_vec_size, l):
         raise ValueError("SFB must be the (32,4,n_tiles,4,k_tiles,L) view over dense atom storage")
-    if tuple(c.shape) != (m, n, l):
+    if c.shape != (m, n, l):
         raise ValueError(f"out must have shape {(m, n, l)}, got {tuple(c.shape)}")
-    if c.stride(1) != 1 or (l > 1 and c.stride(2) != m * n) or (m > 1 and c.stride(0) < n):
+    c_m, c_n, c_l = c.stride()
+    if c_n != 1 or (l > 1 and c_l != m * n) or (m > 1 and c_m < n):
         raise ValueError(f"out must be backed by physical [L, M, N] storage, got strides {c.stride()}")
     if alpha is not None and (alpha.dtype != torch.float32 or alpha.numel() != 1):
         raise ValueError("alpha must be a float32 tensor with one element")
@@ -128,23 +138,17 @@ def _dense_gemm_launch_flat(a, b, sfa, sfb, c, alpha, *, n: int, k: int, l: int,
     block_n = mma_tile_n if mma_tile_n in _KERNEL_BLOCK_N else 0
     if mma_tile_m == 256 and mma_tile_n == 256:
         block_n = _native.BLOCK_N_PAIR
-    k_tiles = -(-(-(-k // sf_vec_size)) // 4)
-    sfa_group = (-(-m // 128)) * k_tiles * 512
-    sfb_group = (-(-n // 128)) * k_tiles * 512
-    sfa_flat = sfa.view(torch.uint8) if sfa.dtype != torch.uint8 else sfa
-    sfb_flat = sfb.view(torch.uint8) if sfb.dtype != torch.uint8 else sfb
-    sfa_base = torch.as_strided(sfa_flat, (l * sfa_group,), (1,))
-    sfb_base = torch.as_strided(sfb_flat, (l * sfb_group,), (1,))
-    ldc = c.stride(0) if m > 1 else n
+    ldc = c_m if m > 1 else n
     if l > 1 and ldc != n:
         raise ValueError("a grouped output must be dense [L, M, N] storage")
+    # The canonical scale views start at their first atom, so the launcher takes them as they are.
     # One launch for all L groups: the operands are physical [L, rows, K] stacks, and the tiles
     # of every group go into one work list on the device. Quantized C: group g fills columns
     # [g * N, (g + 1) * N) of the [M, N * L] MXFP8 matrix.
     qc = None if quantized_c is None else launch.QuantizedC(
         quantized_c[0], quantized_c[1], quantized_c[2], col0=0, total_cols=n * l)
     launch.gemm_blockscaled(
-        kind, a, sfa_base, b, sfb_base, c, None if alpha_is_one else alpha, m, n, k, ldc=ldc,
+        kind, a, sfa, b, sfb, c, None if alpha_is_one else alpha, m, n, k, ldc=ldc,
         block_n=block_n, sm_count=sm_count, stream_int=stream_int, quantized_c=qc, groups=l)
 
 
@@ -367,8 +371,6 @@ def dense_gemm(
     if alpha_dtype is None:
         alpha_dtype = "float32" if alpha is None else str(alpha.dtype).split(".")[-1]
     alpha_is_one = alpha is None
-    if alpha is None:
-        alpha = _cached_alpha_one(a_torch.device)
     stream_int = cuda_stream_to_int(stream)
     if _quantized_c is not None:
         # The GEMM also emits the MXFP8 re-quantization of its BF16 output rows (the decode
@@ -393,12 +395,6 @@ def dense_gemm(
             alpha_is_one=alpha_is_one, stream_int=stream_int,
             quantized_c=(q_values, q_scale_rows, q_scale_mma))
         return out
-    op_tail = (
-        alpha_dtype, sf_vec_size, mma_k, sf_vec_size * 8 if ab_dtype == "float4_e2m1fn" else 128,
-        int(mma_tiler_mn[0]), int(mma_tiler_mn[1]), int(cluster_shape_mn[0]),
-        int(cluster_shape_mn[1]), int(sm_count), False, False, False, 1, False, False,
-        load_path or "tma", bool(swap_ab), bool(sfb_k_replicated), alpha_is_one, stream_int,
-    )
     t0 = time.perf_counter() if _B12X_TIMING else 0.0
     if _direct_launch_ok(a_torch):
         # Plain eager call on real CUDA tensors: what the custom op's body would do, without the
@@ -413,16 +409,25 @@ def dense_gemm(
             sf_dtype=sf_dtype, sf_vec_size=sf_vec_size, mma_tile_n=int(mma_tiler_mn[1]),
             sm_count=int(sm_count), alpha_is_one=alpha_is_one, stream_int=stream_int,
             mma_tile_m=int(mma_tiler_mn[0]))
-    elif out is None:
-        out = torch.ops.b12x.dense_gemm_launch_functional(
-            a_torch, b_torch, sfa_torch, sfb_torch, alpha, n, k, l, l, ab_dtype, sf_dtype,
-            c_dtype, c_dtype, *op_tail)
     else:
-        if out.dtype != _C_DTYPES[c_dtype]:
-            raise ValueError(f"out dtype {out.dtype} does not match c_dtype={c_dtype!r}")
-        torch.ops.b12x.dense_gemm_launch(
-            a_torch, b_torch, sfa_torch, sfb_torch, out, alpha, n, k, l, l, ab_dtype, sf_dtype,
-            c_dtype, *op_tail)
+        if alpha is None:
+            alpha = _cached_alpha_one(a_torch.device)
+        op_tail = (
+            alpha_dtype, sf_vec_size, mma_k, sf_vec_size * 8 if ab_dtype == "float4_e2m1fn" else 128,
+            int(mma_tiler_mn[0]), int(mma_tiler_mn[1]), int(cluster_shape_mn[0]),
+            int(cluster_shape_mn[1]), int(sm_count), False, False, False, 1, False, False,
+            load_path or "tma", bool(swap_ab), bool(sfb_k_replicated), alpha_is_one, stream_int,
+        )
+        if out is None:
+            out = torch.ops.b12x.dense_gemm_launch_functional(
+                a_torch, b_torch, sfa_torch, sfb_torch, alpha, n, k, l, l, ab_dtype, sf_dtype,
+                c_dtype, c_dtype, *op_tail)
+        else:
+            if out.dtype != _C_DTYPES[c_dtype]:
+                raise ValueError(f"out dtype {out.dtype} does not match c_dtype={c_dtype!r}")
+            torch.ops.b12x.dense_gemm_launch(
+                a_torch, b_torch, sfa_torch, sfb_torch, out, alpha, n, k, l, l, ab_dtype, sf_dtype,
+                c_dtype, *op_tail)
     if _B12X_TIMING:
         ms = (time.perf_counter() - t0) * 1000.0
         if ms >= _B12X_TIMING_THRESHOLD_MS:
@@ -445,7 +450,8 @@ def _fused_quant_rhs(name: str, b: torch.Tensor, sfb: torch.Tensor, row_bytes: i
         raise ValueError(f"B must have shape [N,{row_bytes},1], got {tuple(b.shape)}")
     if b.element_size() != 1 or b.stride(1) != 1 or b.stride(0) != row_bytes:
         raise ValueError(f"{name}: B must be K-major one-byte codes")
-    return b.select(2, 0), (sfb.view(torch.uint8) if sfb.dtype != torch.uint8 else sfb)
+    # One-byte scales are passed on as they are (only their address is used).
+    return b, (sfb.view(torch.uint8) if sfb.element_size() != 1 else sfb)
 
 
 def dense_gemm_fused_quant_a(
@@ -487,8 +493,8 @@ def dense_gemm_fused_quant_a(
     if out.shape != (m, n, 1) or out.dtype != torch.bfloat16:
         raise ValueError(
             f"out must be BF16 with shape {(m, n, 1)}, got {out.dtype} {tuple(out.shape)}")
-    launch.gemm_smallm_fused_quant(_native.KIND_MXFP8, source, None, w, sfw, out.select(2, 0),
-                                   None, m, n, k, ldc=n, stream_int=cuda_stream_to_int(stream))
+    launch.gemm_smallm_fused_quant(_native.KIND_MXFP8, source, None, w, sfw, out, None, m, n, k,
+                                   ldc=n, stream_int=cuda_stream_to_int(stream))
     return out
 
 
@@ -608,9 +614,8 @@ def dense_gemm_fused_quant_a_nvfp4(
     if out.shape != (m, n, 1) or out.dtype != _C_DTYPES[c_dtype]:
         raise ValueError(f"out must be {c_dtype} with shape {(m, n, 1)}, got {out.dtype} "
                          f"{tuple(out.shape)}")
-    launch.gemm_smallm_fused_quant(_native.KIND_NVFP4, source, global_scale, w, sfw,
-                                   out.select(2, 0), alpha, m, n, k, ldc=n,
-                                   stream_int=cuda_stream_to_int(stream))
+    launch.gemm_smallm_fused_quant(_native.KIND_NVFP4, source, global_scale, w, sfw, out, alpha,
+                                   m, n, k, ldc=n, stream_int=cuda_stream_to_int(stream))
     return out
 
 

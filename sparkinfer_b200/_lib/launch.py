@@ -8,11 +8,18 @@ of :mod:`sparkinfer_b200._native` raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 from threading import Lock
 
 import torch
 
 from .. import _native
+
+# torch's own accessors without their Python wrappers: at a few microseconds per kernel the host
+# time of a call is most of a decode step, and each wrapper costs as much as a whole check here.
+_current_device = torch._C._cuda_getDevice
+_current_raw_stream = torch._C._cuda_getCurrentRawStream
+_capturing = torch._C._cuda_isCurrentStreamCapturing
 
 _STATUS_LOCK = Lock()
 _STATUS: dict[int, torch.Tensor] = {}
@@ -25,6 +32,8 @@ _WORKSPACES: dict[tuple[int, int], list[torch.Tensor]] = {}
 # which inside a capture would add a fill node to every replay.
 _SPARE_WORKSPACES: dict[int, list[torch.Tensor]] = {}
 _SPARES_PER_DEVICE = 2
+# device index -> size of the smallest spare while all _SPARES_PER_DEVICE are there (else absent).
+_SPARE_BYTES: dict[int, int] = {}
 SMALL_M_MAX = 128        # largest M the decode kernel accepts
 SMALL_M_AUTO = 64        # largest M always routed to it
 FUSED_QUANT_MAX_M = 16   # largest M of the decode kernel with the activation quantizer fused in
@@ -66,10 +75,40 @@ def cuda_stream_to_int(stream: object | None) -> int | None:
     return int(handle) if handle is not None else int(stream)
 
 
-def _stream_ptr(stream_int: int | None, device: torch.device) -> ctypes.c_void_p:
-    if stream_int is None:
-        stream_int = torch.cuda.current_stream(device).cuda_stream
-    return ctypes.c_void_p(int(stream_int))
+def _index_of(device: torch.device) -> int:
+    return device.index if device.index is not None else torch.cuda.current_device()
+
+
+def _stream_ptr(stream_int: int | None, index: int) -> int:
+    """Raw handle of ``stream_int``, by default of torch's current stream on device ``index``."""
+    return _current_raw_stream(index) if stream_int is None else int(stream_int)
+
+
+def _call_on(index: int, fn, *args) -> int:
+    """``fn(*args)`` with device ``index`` current (a device switch costs more than a launch, and
+    the device is nearly always current already)."""
+    if _current_device() == index:
+        return fn(*args)
+    with torch.cuda.device(index):
+        return fn(*args)
+
+
+def plain_eager(*tensors: torch.Tensor | None) -> bool:
+    """Whether a call on these tensors can go straight to the launcher: ordinary CUDA tensors with
+    nothing that listens to operators (tracing, dispatch modes, functorch transforms, forward-mode
+    differentiation, a graph being recorded for one of them). Otherwise it belongs to the
+    registered custom op, which all of these know how to treat."""
+    if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() != 0
+            or torch._C._get_tracing_state() is not None
+            or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch.autograd.forward_ad._current_level >= 0):
+        return False
+    grad = torch.is_grad_enabled()
+    for t in tensors:
+        if t is not None and ((type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter)
+                              or not t.is_cuda or (grad and t.requires_grad)):
+            return False
+    return True
 
 
 def _zeros_ready_for_any_stream(nbytes: int, index: int, dtype=torch.uint8) -> torch.Tensor:
@@ -90,12 +129,20 @@ def _top_up_spares(index: int, size: int) -> None:
     spares[:] = [b for b in spares if b.numel() >= size]
     while len(spares) < _SPARES_PER_DEVICE:
         spares.append(_zeros_ready_for_any_stream(size, index))
+    _SPARE_BYTES[index] = min(b.numel() for b in spares)
 
 
 def status_buffer(device: torch.device) -> torch.Tensor:
     """Per-device int32[4] the kernels raise when a bounded wait runs out. Allocated once, on
     first use (call an op once before CUDA-graph capture, as with any warm-up)."""
     index = device.index if device.index is not None else torch.cuda.current_device()
+    return _status_of(index)
+
+
+def _status_of(index: int) -> torch.Tensor:
+    buf = _STATUS.get(index)
+    if buf is not None:
+        return buf
     with _STATUS_LOCK:
         buf = _STATUS.get(index)
         if buf is None:
@@ -140,10 +187,19 @@ def stream_workspace(need: int, device: torch.device, stream_int: int | None = N
     buffer is created zeroed the first time a stream needs one, or a larger one (so warm up
     before CUDA-graph capture), and is never released while the process lives."""
     index = device.index if device.index is not None else torch.cuda.current_device()
-    if stream_int is None:
-        stream_int = torch.cuda.current_stream(torch.device("cuda", index)).cuda_stream
-    key = (index, int(stream_int))
-    capturing = torch.cuda.is_current_stream_capturing()
+    return _workspace_of(need, index, _stream_ptr(stream_int, index))
+
+
+def _workspace_of(need: int, index: int, stream: int) -> torch.Tensor:
+    key = (index, stream)
+    capturing = _capturing()
+    # Nothing to create and no spare to replace: the list is only ever appended to, so reading its
+    # last entry needs no lock.
+    known = _WORKSPACES.get(key)
+    if known:
+        last = known[-1]
+        if last.numel() >= need and (capturing or _SPARE_BYTES.get(index, 0) >= last.numel()):
+            return last
     with _STATUS_LOCK:
         bufs = _WORKSPACES.setdefault(key, [])
         if not bufs or bufs[-1].numel() < need:
@@ -154,6 +210,7 @@ def stream_workspace(need: int, device: torch.device, stream_int: int | None = N
             fit = next((b for b in spares if b.numel() >= size), None) if capturing else None
             if fit is not None:
                 spares[:] = [b for b in spares if b is not fit]
+                _SPARE_BYTES.pop(index, None)
                 bufs.append(fit)
             else:
                 bufs.append(_zeros_ready_for_any_stream(size, index))
@@ -166,11 +223,23 @@ def smallm_workspace(kind: int, m: int, n: int, k: int, device: torch.device,
                      sm_count: int = 0, stream_int: int | None = None) -> torch.Tensor:
     """:func:`stream_workspace` sized for the decode-shape kernel on (M, N, K)."""
     index = device.index if device.index is not None else torch.cuda.current_device()
-    with torch.cuda.device(index):
-        need = int(_native.load().b12x_b200_gemm_smallm_workspace_bytes(kind, m, n, k, sm_count))
+    need = _workspace_need(index, kind, 1, m, n, k, 1, 0, sm_count)
+    return _workspace_of(need, index, _stream_ptr(stream_int, index))
+
+
+@functools.lru_cache(maxsize=4096)
+def _workspace_need(index: int, kind: int, decode: int, m: int, n: int, k: int, groups: int,
+                    block_n: int, sm_count: int) -> int:
+    """Scratch bytes of a GEMM (a function of the sizes and the device alone): counters and partial
+    tiles of the decode kernel, or what the CTA-pair kernel's split leftover tiles need (0 when
+    the shape has none)."""
+    need = int(_call_on(index, _native.load().b12x_b200_gemm_grouped_workspace_bytes, kind, decode,
+                        m, n, k, groups, block_n, sm_count))
     if need < 0:
-        raise _native.NativeLibraryError(f"no decode-shape plan for M={m}, N={n}, K={k}")
-    return stream_workspace(need, device, stream_int)
+        what = "decode-shape" if decode else "kernel"
+        raise _native.NativeLibraryError(
+            f"no {what} plan for M={m}, N={n}, K={k}" + (f", groups={groups}" if groups != 1 else ""))
+    return need
 
 
 def route_to_decode_kernel(m: int, n: int, device: torch.device, sm_count: int = 0) -> bool:
@@ -236,11 +305,16 @@ def gemm_blockscaled(kind: int, a: torch.Tensor, sfa: torch.Tensor | None, b: to
     with ``small_m=True``) go to the weight-streaming stream-K kernel, everything else to the
     persistent tiled kernels; ``block_n=_native.BLOCK_N_PAIR`` forces the CTA-pair kernel."""
     plain = kind == _native.KIND_FP8      # no block scales: sfa / sfb are not read
-    for name, t in (("a", a), ("b", b), ("c", c)) + (() if plain else (("sfa", sfa), ("sfb", sfb))):
-        _require_cuda(name, t)
-    if c.dtype not in _DTYPE_CODE:
+    _require_cuda("a", a)
+    _require_cuda("b", b)
+    _require_cuda("c", c)
+    if not plain:
+        _require_cuda("sfa", sfa)
+        _require_cuda("sfb", sfb)
+    dtype_code = _DTYPE_CODE.get(c.dtype)
+    if dtype_code is None:
         raise TypeError(f"unsupported output dtype {c.dtype}")
-    dev = a.device
+    index = a.get_device()
     ep = _epilogue(c, n, bias, quantized_c)
     if plain:
         if small_m or quantized_c is not None:
@@ -248,36 +322,30 @@ def gemm_blockscaled(kind: int, a: torch.Tensor, sfa: torch.Tensor | None, b: to
         small_m = False
     if small_m is None:
         small_m = block_n == 0 and 0 < m <= SMALL_M_MAX and (
-            quantized_c is not None or route_to_decode_kernel(m, n, dev, sm_count))
+            quantized_c is not None or route_to_decode_kernel(m, n, a.device, sm_count))
     lib = _native.load()
     decode = bool(small_m and 0 < m <= SMALL_M_MAX and n > 0)
-    with torch.cuda.device(dev):
-        # Decode kernel: counters and partial tiles. Tiled kernels: scratch for the CTA-pair
-        # kernel's split leftover tiles (0 when the shape has none).
-        need = int(lib.b12x_b200_gemm_grouped_workspace_bytes(
-            kind, int(decode), m, n, k, groups, 0 if decode else block_n, sm_count))
-    if need < 0:
-        raise _native.NativeLibraryError(f"no kernel plan for M={m}, N={n}, K={k}, groups={groups}")
-    work = stream_workspace(need, dev, stream_int) if need > 0 else None
-    common_tail = (work.data_ptr() if work is not None else None,
-                   work.numel() if work is not None else 0,
-                   ctypes.byref(ep) if ep is not None else None)
+    stream = _stream_ptr(stream_int, index)
+    need = _workspace_need(index, kind, 1 if decode else 0, m, n, k, groups,
+                           0 if decode else block_n, sm_count)
+    work = _workspace_of(need, index, stream) if need > 0 else None
+    work_ptr, work_bytes = (work.data_ptr(), work.numel()) if work is not None else (None, 0)
+    ep_ref = ctypes.byref(ep) if ep is not None else None
     head = (kind, a.data_ptr(), None if plain else sfa.data_ptr(), b.data_ptr(),
-            None if plain else sfb.data_ptr(), c.data_ptr(),
-            _DTYPE_CODE[c.dtype], alpha.data_ptr() if alpha is not None else None,
+            None if plain else sfb.data_ptr(), c.data_ptr(), dtype_code,
+            alpha.data_ptr() if alpha is not None else None,
             m, n, k, ldc if ldc is not None else n, groups)
-    with torch.cuda.device(dev):
-        if decode:
-            rc = lib.b12x_b200_gemm_blockscaled_smallm_grouped(
-                *head, *common_tail, sm_count, status_buffer(dev).data_ptr(),
-                _stream_ptr(stream_int, dev))
-        else:
-            rc = lib.b12x_b200_gemm_blockscaled_grouped(
-                *head, block_n, sm_count, *common_tail, status_buffer(dev).data_ptr(),
-                _stream_ptr(stream_int, dev))
-    _native.check(rc, "b12x_b200_gemm_blockscaled_smallm_grouped" if decode
-                  else "b12x_b200_gemm_blockscaled_grouped")
-    _after_launch(dev)
+    if decode:
+        rc = _call_on(index, lib.b12x_b200_gemm_blockscaled_smallm_grouped, *head, work_ptr,
+                      work_bytes, ep_ref, sm_count, _status_of(index).data_ptr(), stream)
+    else:
+        rc = _call_on(index, lib.b12x_b200_gemm_blockscaled_grouped, *head, block_n, sm_count,
+                      work_ptr, work_bytes, ep_ref, _status_of(index).data_ptr(), stream)
+    if rc != 0:
+        _native.check(rc, "b12x_b200_gemm_blockscaled_smallm_grouped" if decode
+                      else "b12x_b200_gemm_blockscaled_grouped")
+    if _CHECK_AFTER_LAUNCH:
+        _after_launch(a.device)
 
 
 def gemm_smallm_fused_quant(kind: int, x: torch.Tensor, global_scale: torch.Tensor | None,
@@ -292,26 +360,22 @@ def gemm_smallm_fused_quant(kind: int, x: torch.Tensor, global_scale: torch.Tens
     ``groups > 1``: ``x [M, groups, K]``, weights / scale atoms / output group-major, one
     launch. ``inv_rope = (positions, cos_sin_cache, head_dim, nope_dim, rope_dim)`` (MXFP8
     only) rotates the rotary part of every head back before the rows are quantized."""
-    for name, t in (("x", x), ("w", w), ("sfw", sfw), ("c", c)):
-        _require_cuda(name, t)
+    _require_cuda("x", x)
+    _require_cuda("w", w)
+    _require_cuda("sfw", sfw)
+    _require_cuda("c", c)
     if x.dtype != torch.bfloat16 or x.stride(-1) != 1:
         raise ValueError("fused activation quantization needs BF16 rows with unit column stride")
     if c.dtype not in _DTYPE_CODE:
         raise TypeError(f"unsupported output dtype {c.dtype}")
-    dev = x.device
+    index = x.get_device()
     ep = _epilogue(c, n, bias, quantized_c)
+    stream = _stream_ptr(stream_int, index)
+    work = _workspace_of(_workspace_need(index, kind, 1, m, n, k, groups, 0, sm_count), index, stream)
     if groups == 1:
-        work = smallm_workspace(kind, m, n, k, dev, sm_count, stream_int)
         row_stride, group_stride = (x.stride(0) if m > 1 else k), 0
     else:
         # x is [M, groups, K]: rows `x.stride(0)` apart, groups `x.stride(1)` apart.
-        with torch.cuda.device(dev):
-            need = int(_native.load().b12x_b200_gemm_grouped_workspace_bytes(
-                kind, 1, m, n, k, groups, 0, sm_count))
-        if need < 0:
-            raise _native.NativeLibraryError(
-                f"no decode-shape plan for M={m}, N={n}, K={k}, groups={groups}")
-        work = stream_workspace(need, dev, stream_int)
         row_stride, group_stride = (x.stride(0) if m > 1 else groups * k), x.stride(1)
     if inv_rope is not None:
         positions, cache, head_dim, nope_dim, rope_dim = inv_rope
@@ -319,29 +383,31 @@ def gemm_smallm_fused_quant(kind: int, x: torch.Tensor, global_scale: torch.Tens
         _require_cuda("cos_sin_cache", cache)
         if kind != _native.KIND_MXFP8 or ep is not None:
             raise ValueError("the inverse-RoPE prologue exists for MXFP8 without epilogue only")
-        with torch.cuda.device(dev):
-            rc = _native.load().b12x_b200_gemm_smallm_fused_quant_grouped_inv_rope(
-                x.data_ptr(), row_stride, group_stride, positions.data_ptr(),
-                1 if positions.dtype == torch.int64 else 0, cache.data_ptr(),
-                1 if cache.dtype == torch.float32 else 0, head_dim, nope_dim, rope_dim,
-                w.data_ptr(), sfw.data_ptr(), c.data_ptr(), _DTYPE_CODE[c.dtype],
-                alpha.data_ptr() if alpha is not None else None, m, n, k,
-                ldc if ldc is not None else n, groups, work.data_ptr(), work.numel(), sm_count,
-                status_buffer(dev).data_ptr(), _stream_ptr(stream_int, dev))
-        _native.check(rc, "b12x_b200_gemm_smallm_fused_quant_grouped_inv_rope")
-        _after_launch(dev)
-        return
-    with torch.cuda.device(dev):
-        rc = _native.load().b12x_b200_gemm_smallm_fused_quant_grouped(
-            kind, x.data_ptr(), row_stride, group_stride,
-            global_scale.data_ptr() if global_scale is not None else None, w.data_ptr(),
-            sfw.data_ptr(), c.data_ptr(), _DTYPE_CODE[c.dtype],
+        rc = _call_on(
+            index, _native.load().b12x_b200_gemm_smallm_fused_quant_grouped_inv_rope,
+            x.data_ptr(), row_stride, group_stride, positions.data_ptr(),
+            1 if positions.dtype == torch.int64 else 0, cache.data_ptr(),
+            1 if cache.dtype == torch.float32 else 0, head_dim, nope_dim, rope_dim,
+            w.data_ptr(), sfw.data_ptr(), c.data_ptr(), _DTYPE_CODE[c.dtype],
             alpha.data_ptr() if alpha is not None else None, m, n, k,
-            ldc if ldc is not None else n, groups, work.data_ptr(), work.numel(),
-            ctypes.byref(ep) if ep is not None else None, sm_count,
-            status_buffer(dev).data_ptr(), _stream_ptr(stream_int, dev))
-    _native.check(rc, "b12x_b200_gemm_smallm_fused_quant_grouped")
-    _after_launch(dev)
+            ldc if ldc is not None else n, groups, work.data_ptr(), work.numel(), sm_count,
+            _status_of(index).data_ptr(), stream)
+        _native.check(rc, "b12x_b200_gemm_smallm_fused_quant_grouped_inv_rope")
+        _after_launch(x.device)
+        return
+    rc = _call_on(
+        index, _native.load().b12x_b200_gemm_smallm_fused_quant_grouped,
+        kind, x.data_ptr(), row_stride, group_stride,
+        global_scale.data_ptr() if global_scale is not None else None, w.data_ptr(),
+        sfw.data_ptr(), c.data_ptr(), _DTYPE_CODE[c.dtype],
+        alpha.data_ptr() if alpha is not None else None, m, n, k,
+        ldc if ldc is not None else n, groups, work.data_ptr(), work.numel(),
+        ctypes.byref(ep) if ep is not None else None, sm_count,
+        _status_of(index).data_ptr(), stream)
+    if rc != 0:
+        _native.check(rc, "b12x_b200_gemm_smallm_fused_quant_grouped")
+    if _CHECK_AFTER_LAUNCH:
+        _after_launch(x.device)
 
 
 def gemm_smallm_timeline(kind: int, a: torch.Tensor, sfa: torch.Tensor, b: torch.Tensor,
@@ -356,7 +422,7 @@ def gemm_smallm_timeline(kind: int, a: torch.Tensor, sfa: torch.Tensor, b: torch
             kind, a.data_ptr(), sfa.data_ptr(), b.data_ptr(), sfb.data_ptr(), c.data_ptr(),
             _DTYPE_CODE[c.dtype], alpha.data_ptr() if alpha is not None else None, m, n, k, n,
             work.data_ptr(), work.numel(), 0, stamps.data_ptr(), stamps.numel(),
-            status_buffer(dev).data_ptr(), _stream_ptr(stream_int, dev))
+            status_buffer(dev).data_ptr(), _stream_ptr(stream_int, _index_of(dev)))
     _native.check(rc, "b12x_b200_gemm_smallm_timeline")
 
 
@@ -365,7 +431,7 @@ def selftest_wait_timeout(device: torch.device, max_polls: int = 4096) -> None:
     device's status word like a GEMM kernel would (see :func:`check_kernel_status`)."""
     with torch.cuda.device(device):
         rc = _native.load().b12x_b200_selftest_wait_timeout(
-            status_buffer(device).data_ptr(), max_polls, _stream_ptr(None, device))
+            status_buffer(device).data_ptr(), max_polls, _stream_ptr(None, _index_of(device)))
     _native.check(rc, "b12x_b200_selftest_wait_timeout")
 
 
@@ -374,44 +440,51 @@ def gemm_block_fp8(a: torch.Tensor, sfa: torch.Tensor, b: torch.Tensor, sfb: tor
                    ldc: int | None = None, sm_count: int = 0,
                    stream_int: int | None = None, bias: torch.Tensor | None = None) -> None:
     """E4M3 operands with FP32 scales ``sfa [M, K/128]`` / ``sfb [N/128, K/128]``."""
-    for name, t in (("a", a), ("b", b), ("sfa", sfa), ("sfb", sfb), ("c", c)):
-        _require_cuda(name, t)
-    dev = a.device
+    _require_cuda("a", a)
+    _require_cuda("b", b)
+    _require_cuda("sfa", sfa)
+    _require_cuda("sfb", sfb)
+    _require_cuda("c", c)
+    index = a.get_device()
     ep = _epilogue(c, n, bias, None)
-    with torch.cuda.device(dev):
-        rc = _native.load().b12x_b200_gemm_block_fp8_ex(
-            a.data_ptr(), sfa.data_ptr(), b.data_ptr(), sfb.data_ptr(), c.data_ptr(),
-            _DTYPE_CODE[c.dtype], alpha.data_ptr() if alpha is not None else None, m, n, k,
-            ldc if ldc is not None else n, sm_count, ctypes.byref(ep) if ep is not None else None,
-            status_buffer(dev).data_ptr(), _stream_ptr(stream_int, dev))
-    _native.check(rc, "b12x_b200_gemm_block_fp8_ex")
-    _after_launch(dev)
+    rc = _call_on(
+        index, _native.load().b12x_b200_gemm_block_fp8_ex,
+        a.data_ptr(), sfa.data_ptr(), b.data_ptr(), sfb.data_ptr(), c.data_ptr(),
+        _DTYPE_CODE[c.dtype], alpha.data_ptr() if alpha is not None else None, m, n, k,
+        ldc if ldc is not None else n, sm_count, ctypes.byref(ep) if ep is not None else None,
+        _status_of(index).data_ptr(), _stream_ptr(stream_int, index))
+    if rc != 0:
+        _native.check(rc, "b12x_b200_gemm_block_fp8_ex")
+    if _CHECK_AFTER_LAUNCH:
+        _after_launch(a.device)
 
 
 def quantize_mxfp8_rows(src: torch.Tensor, values: torch.Tensor, scale_rows: torch.Tensor | None,
                         scale_mma: torch.Tensor | None, *, stream_int: int | None = None) -> None:
     _require_cuda("source", src)
     m, k = src.shape
-    dev = src.device
-    with torch.cuda.device(dev):
-        rc = _native.load().b12x_b200_quantize_mxfp8_rows(
-            src.data_ptr(), _DTYPE_CODE[src.dtype], src.stride(0), values.data_ptr(),
-            scale_rows.data_ptr() if scale_rows is not None else None,
-            scale_mma.data_ptr() if scale_mma is not None else None, m, k,
-            _stream_ptr(stream_int, dev))
-    _native.check(rc, "b12x_b200_quantize_mxfp8_rows")
+    index = src.get_device()
+    rc = _call_on(
+        index, _native.load().b12x_b200_quantize_mxfp8_rows,
+        src.data_ptr(), _DTYPE_CODE[src.dtype], src.stride(0), values.data_ptr(),
+        scale_rows.data_ptr() if scale_rows is not None else None,
+        scale_mma.data_ptr() if scale_mma is not None else None, m, k,
+        _stream_ptr(stream_int, index))
+    if rc != 0:
+        _native.check(rc, "b12x_b200_quantize_mxfp8_rows")
 
 
 def quantize_nvfp4_rows(src: torch.Tensor, global_scale: torch.Tensor, packed: torch.Tensor,
                         scale_mma: torch.Tensor, *, stream_int: int | None = None) -> None:
     _require_cuda("source", src)
     m, k = src.shape
-    dev = src.device
-    with torch.cuda.device(dev):
-        rc = _native.load().b12x_b200_quantize_nvfp4_rows(
-            src.data_ptr(), _DTYPE_CODE[src.dtype], src.stride(0), global_scale.data_ptr(),
-            packed.data_ptr(), scale_mma.data_ptr(), m, k, _stream_ptr(stream_int, dev))
-    _native.check(rc, "b12x_b200_quantize_nvfp4_rows")
+    index = src.get_device()
+    rc = _call_on(
+        index, _native.load().b12x_b200_quantize_nvfp4_rows,
+        src.data_ptr(), _DTYPE_CODE[src.dtype], src.stride(0), global_scale.data_ptr(),
+        packed.data_ptr(), scale_mma.data_ptr(), m, k, _stream_ptr(stream_int, index))
+    if rc != 0:
+        _native.check(rc, "b12x_b200_quantize_nvfp4_rows")
 
 
 def gemm_blockscaled_scatter(kind: int, a: torch.Tensor, sfa: torch.Tensor | None, b: torch.Tensor,
@@ -440,7 +513,7 @@ def gemm_blockscaled_scatter(kind: int, a: torch.Tensor, sfa: torch.Tensor | Non
             _DTYPE_CODE[dtype], alpha.data_ptr() if alpha is not None else None, m, n, k,
             ld if ld is not None else n, sm_count, work.data_ptr() if work is not None else None,
             work.numel() if work is not None else 0, status_buffer(dev).data_ptr(),
-            _stream_ptr(stream_int, dev))
+            _stream_ptr(stream_int, _index_of(dev)))
     _native.check(rc, "b12x_b200_gemm_blockscaled_scatter")
     _after_launch(dev)
 
@@ -461,7 +534,7 @@ def pack_block_fp8_weight_mxfp8(codes: torch.Tensor, scale: torch.Tensor, out_co
             codes.data_ptr(), scale.data_ptr(), out_codes.data_ptr(),
             scale_rows.data_ptr() if scale_rows is not None else None,
             scale_mma.data_ptr() if scale_mma is not None else None, m, k, groups,
-            1 if requantize else 0, _stream_ptr(stream_int, dev))
+            1 if requantize else 0, _stream_ptr(stream_int, _index_of(dev)))
     _native.check(rc, "b12x_b200_pack_block_fp8_weight_mxfp8")
 
 
@@ -471,17 +544,20 @@ def bmm_mxfp8(a: torch.Tensor, w_values: torch.Tensor, w_scales: torch.Tensor, o
     """``out[b] = a[b] @ dequant(w[b])``: BF16 ``a [B, M, K]`` (M <= 32), rowwise-MXFP8 weights
     (``[B, N, K]`` K-major or ``[B, K, N]`` N-major, one UE8M0 byte per 32 codes of the inner
     axis), BF16 ``out [B, M, N]``. The tensors may be strided views; inner axes are contiguous."""
-    for name, t in (("a", a), ("w_values", w_values), ("w_scales", w_scales), ("out", out)):
-        _require_cuda(name, t)
-    dev = a.device
-    with torch.cuda.device(dev):
-        rc = _native.load().b12x_b200_bmm_mxfp8(
-            a.data_ptr(), a.stride(0), a.stride(1),
-            w_values.data_ptr(), w_values.stride(0), w_values.stride(1),
-            w_scales.data_ptr(), w_scales.stride(0), w_scales.stride(1),
-            out.data_ptr(), out.stride(0), out.stride(1), 1 if n_major else 0,
-            batch, m, n, k, _stream_ptr(stream_int, dev))
-    _native.check(rc, "b12x_b200_bmm_mxfp8")
+    _require_cuda("a", a)
+    _require_cuda("w_values", w_values)
+    _require_cuda("w_scales", w_scales)
+    _require_cuda("out", out)
+    index = a.get_device()
+    (a0, a1, _), (v0, v1, _) = a.stride(), w_values.stride()
+    (s0, s1, _), (o0, o1, _) = w_scales.stride(), out.stride()
+    rc = _call_on(
+        index, _native.load().b12x_b200_bmm_mxfp8,
+        a.data_ptr(), a0, a1, w_values.data_ptr(), v0, v1, w_scales.data_ptr(), s0, s1,
+        out.data_ptr(), o0, o1, 1 if n_major else 0,
+        batch, m, n, k, _stream_ptr(stream_int, index))
+    if rc != 0:
+        _native.check(rc, "b12x_b200_bmm_mxfp8")
 
 
 def allreduce_peer_signal_bytes() -> int:
@@ -508,13 +584,13 @@ def allreduce_peer(buffer_ptrs: list[int], signal_ptrs: list[int], rank: int, dt
         if output_ptrs is None:
             name = "b12x_b200_allreduce_peer"
             rc = _native.load().b12x_b200_allreduce_peer(
-                bufs, sigs, *tail, status_buffer(device).data_ptr(), _stream_ptr(stream_int, device))
+                bufs, sigs, *tail, status_buffer(device).data_ptr(), _stream_ptr(stream_int, _index_of(device)))
         else:
             name = "b12x_b200_allreduce_peer_scattered"
             outs = (ctypes.c_void_p * world)(*output_ptrs)
             rc = _native.load().b12x_b200_allreduce_peer_scattered(
                 bufs, outs, sigs, *tail, status_buffer(device).data_ptr(),
-                _stream_ptr(stream_int, device))
+                _stream_ptr(stream_int, _index_of(device)))
     _native.check(rc, name)
     _after_launch(device)
 

@@ -86,14 +86,13 @@ def mma_view_is_canonical(sf: torch.Tensor, m: int, k: int, sf_vec_size: int,
     """True when ``sf`` is the 6-D permuted view over dense ``[L][mt][kt][32][4][4]`` bytes
     (or a flat / contiguous tensor of exactly that many bytes)."""
     shape = get_mma_sf_shape(m, k, num_groups, sf_vec_size)
-    nbytes = math.prod(shape)
     if sf.element_size() != 1:
         return False
-    if sf.ndim == 6 and tuple(sf.shape) == shape:
-        _, _, m_tiles, _, k_tiles, _ = shape
-        want = (16, 4, k_tiles * 512, 1, 512, m_tiles * k_tiles * 512)
-        return all(sf.shape[i] == 1 or sf.stride(i) == want[i] for i in range(6))
-    return sf.is_contiguous() and sf.numel() == nbytes
+    _, _, m_tiles, _, k_tiles, _ = shape
+    if sf.shape == shape:
+        have, want = sf.stride(), (16, 4, k_tiles * 512, 1, 512, m_tiles * k_tiles * 512)
+        return have == want or all(n == 1 or h == w for n, h, w in zip(shape, have, want))
+    return sf.is_contiguous() and sf.numel() == m_tiles * k_tiles * 512 * num_groups
 
 
 __all__ = [

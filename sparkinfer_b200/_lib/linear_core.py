@@ -67,7 +67,7 @@ class SourceRows:
         if source.ndim == 0:
             raise ValueError("source must have at least one dimension")
         k = int(source.shape[-1])
-        rows = source.reshape(-1, k)
+        rows = source if source.ndim == 2 else source.reshape(-1, k)
         if copy:
             rows = rows.contiguous()
         if k != int(packed_in_features):
@@ -78,7 +78,8 @@ class SourceRows:
                    leading_shape=tuple(source.shape[:-1]))
 
     def restore(self, output_2d: torch.Tensor, out_features: int) -> torch.Tensor:
-        return output_2d.view(*self.leading_shape, out_features)
+        shape = (*self.leading_shape, out_features)
+        return output_2d if output_2d.shape == shape else output_2d.view(shape)
 
 
 @dataclass(frozen=True)
@@ -144,13 +145,10 @@ def mxfp8_gemm(x_q: MXFP8Rows, weight_values: torch.Tensor, weight_scale_mma: to
                tokens: int, k: int, out_features: int, out: torch.Tensor,
                bias: torch.Tensor | None, stream: object) -> None:
     """``out [T, N, 1] = x_q @ W^T (+ bias)`` on MXFP8 rows, straight through the launcher."""
-    atoms = x_q.scale_mma
     launch.gemm_blockscaled(
-        _native.KIND_MXFP8, x_q.values, atoms.view(torch.uint8) if atoms.dtype != torch.uint8 else atoms,
-        weight_values, weight_scale_mma.view(torch.uint8) if weight_scale_mma.dtype != torch.uint8
-        else weight_scale_mma, out.select(2, 0), None, tokens, out_features, k,
-        ldc=out.stride(0) if tokens > 1 else out_features, stream_int=cuda_stream_to_int(stream),
-        bias=bias)
+        _native.KIND_MXFP8, x_q.values, x_q.scale_mma, weight_values, weight_scale_mma, out, None,
+        tokens, out_features, k, ldc=out.stride(0) if tokens > 1 else out_features,
+        stream_int=cuda_stream_to_int(stream), bias=bias)
 
 
 def quantize_then_gemm(rows: torch.Tensor, weight_values: torch.Tensor,
@@ -166,7 +164,7 @@ def quantize_then_gemm(rows: torch.Tensor, weight_values: torch.Tensor,
     fused = bias_fuses(bias, out.dtype, out_features)
     mxfp8_gemm(x_q, weight_values, weight_scale_mma, tokens=tokens, k=padded_k,
                out_features=out_features, out=out, bias=bias if fused else None, stream=stream)
-    result = out[:, :, 0]
+    result = out.select(2, 0)
     if bias is not None and not fused:
         result = result.add_(bias) if bias_in_place else result + bias
     return result

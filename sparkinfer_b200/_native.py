@@ -173,6 +173,8 @@ def library_path() -> Path:
 def load() -> ctypes.CDLL:
     """Load the shared object once and declare every prototype."""
     global _LIB
+    if _LIB is not None:
+        return _LIB
     with _LOCK:
         if _LIB is not None:
             return _LIB

@@ -55,17 +55,17 @@ def _rhs_geometry(values: torch.Tensor, scales: torch.Tensor, b_major, sf_axis):
     if values.ndim != 3:
         raise ValueError(f"rhs values must be 3-D, got shape {tuple(values.shape)}")
     if major == "n":
-        groups, k, n = (int(s) for s in values.shape)
+        groups, k, n = values.shape
         scale_shape = (groups, k, n // 32)
     else:
-        groups, n, k = (int(s) for s in values.shape)
+        groups, n, k = values.shape
         scale_shape = (groups, n, k // 32)
     if n <= 0 or k <= 0:
         raise ValueError(f"rhs dimensions must be positive, got N={n}, K={k}")
     if int(values.shape[-1]) % 32:
         raise ValueError("rhs physical inner dimension must be divisible by sf_vec_size=32, "
                          f"got {values.shape[-1]}")
-    if tuple(scales.shape) != scale_shape:
+    if scales.shape != scale_shape:
         raise ValueError(f"rhs scales must have shape {scale_shape} for b_major={major!r}, "
                          f"sf_axis={sf_axis!r}; got {tuple(scales.shape)}")
     return major, groups, n, k
@@ -77,12 +77,13 @@ def _qualified(major: str, groups: int, m: int, n: int, k: int) -> bool:
 
 
 def _check_strided(name: str, t: torch.Tensor, *, stride_mod: int, ptr_align: int) -> None:
-    if t.stride(2) != 1:
+    outer, middle, inner = t.stride()
+    if inner != 1:
         raise ValueError(f"{name} physical inner dimension must be contiguous")
-    if t.stride(0) <= 0 or t.stride(1) <= 0:
+    if outer <= 0 or middle <= 0:
         raise ValueError(f"{name} outer strides must be positive, got {t.stride()}")
-    if t.stride(0) % stride_mod or t.stride(1) % stride_mod:
-        raise ValueError(f"{name} outer strides {t.stride(0)}/{t.stride(1)} must be multiples "
+    if outer % stride_mod or middle % stride_mod:
+        raise ValueError(f"{name} outer strides {outer}/{middle} must be multiples "
                          f"of {stride_mod} elements")
     if t.data_ptr() % ptr_align:
         raise ValueError(f"{name} base pointer must be {ptr_align}-byte aligned")
@@ -91,7 +92,7 @@ def _check_strided(name: str, t: torch.Tensor, *, stride_mod: int, ptr_align: in
 def _check_operand(name: str, t: torch.Tensor, shape, *, stride_mod: int, ptr_align: int) -> None:
     if t.dtype != torch.bfloat16:
         raise ValueError(f"{name} must be bfloat16, got {t.dtype}")
-    if tuple(t.shape) != tuple(shape):
+    if t.shape != shape:
         raise ValueError(f"{name} must have shape {tuple(shape)}, got {tuple(t.shape)}")
     _check_strided(name, t, stride_mod=stride_mod, ptr_align=ptr_align)
 
@@ -103,7 +104,7 @@ def _validate_rhs_storage(values: torch.Tensor, scales: torch.Tensor) -> None:
         raise ValueError(f"rhs scales must be uint8/e8m0, got {scales.dtype}")
     if not values.is_cuda or not scales.is_cuda:
         raise ValueError("BMM RHS tensors must be CUDA tensors")
-    if values.device != scales.device:
+    if values.get_device() != scales.get_device():
         raise ValueError("BMM RHS tensors must be on the same CUDA device")
     for name, t, align in (("rhs values", values, 16), ("rhs scales", scales, 4)):
         if t.ndim != 3:
@@ -112,21 +113,19 @@ def _validate_rhs_storage(values: torch.Tensor, scales: torch.Tensor) -> None:
 
 
 def _interval(t: torch.Tensor) -> tuple[int, int]:
+    if t.is_contiguous():
+        start = t.data_ptr()
+        return start, start + t.numel() * t.element_size()
     extent = 1 + sum((int(size) - 1) * int(stride)
                      for size, stride in zip(t.shape, t.stride()) if int(size) > 0)
     start = int(t.data_ptr())
     return start, start + extent * t.element_size()
 
 
-def _overlaps(x: torch.Tensor, y: torch.Tensor) -> bool:
-    if x.device != y.device:
-        return False
-    (x0, x1), (y0, y1) = _interval(x), _interval(y)
-    return max(x0, y0) < min(x1, y1)
-
-
 def _has_internal_overlap(t: torch.Tensor) -> bool:
     """True when two index tuples can reach one element (sizes sorted by stride must nest)."""
+    if t.is_contiguous():
+        return False
     dims = sorted(((int(st), int(sz)) for sz, st in zip(t.shape, t.stride()) if int(sz) > 1))
     reach = 1
     for stride, size in dims:
@@ -140,7 +139,7 @@ def _validate_launch(a, values, scales, out, b_major, sf_axis):
     major, b_groups, n, b_k = _rhs_geometry(values, scales, b_major, sf_axis)
     if a.ndim != 3:
         raise ValueError(f"lhs must have shape [B,M,K], got {tuple(a.shape)}")
-    groups, m, k = (int(s) for s in a.shape)
+    groups, m, k = a.shape
     if groups != b_groups or k != b_k:
         raise ValueError("lhs and rhs batch/K dimensions must match: "
                          f"lhs is [B,M,K]=[{groups},{m},{k}], rhs implies B={b_groups}, K={b_k}")
@@ -149,18 +148,20 @@ def _validate_launch(a, values, scales, out, b_major, sf_axis):
     if _has_internal_overlap(out):
         raise ValueError("out must not have internal storage overlap")
     _validate_rhs_storage(values, scales)
-    tensors = (a, values, scales, out)
-    if not all(t.is_cuda for t in tensors):
+    if not (a.is_cuda and values.is_cuda and scales.is_cuda and out.is_cuda):
         raise ValueError("BMM operands must be CUDA tensors")
-    if any(t.device != a.device for t in tensors[1:]):
+    index = a.get_device()
+    if values.get_device() != index or scales.get_device() != index or out.get_device() != index:
         raise ValueError("BMM operands must be on the same CUDA device")
     if not _qualified(major, groups, m, n, k):
         raise NotImplementedError(
             "the BMM MXFP8 specialization is qualified for b_major='n' [B,K,N]=[16,192,512] or "
             "b_major='k' [B,N,K]=[16,256,512], with 1<=M<=32; "
             f"got b_major={major!r}, B={groups}, M={m}, N={n}, K={k}")
+    out0, out1 = _interval(out)
     for name, source in (("lhs", a), ("rhs values", values), ("rhs scales", scales)):
-        if _overlaps(out, source):
+        begin, end = _interval(source)
+        if max(out0, begin) < min(out1, end):
             raise ValueError(f"out must not overlap {name}")
     return major, groups, m, n, k
 

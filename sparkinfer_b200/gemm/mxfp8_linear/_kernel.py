@@ -9,7 +9,7 @@ from dataclasses import dataclass
 
 import torch
 
-from ..._lib.launch import cuda_stream_to_int
+from ..._lib.launch import cuda_stream_to_int, plain_eager
 from ..._lib.linear_core import (
     K_STEP,
     SourceRows,
@@ -24,8 +24,6 @@ from ..._lib.mxfp8_rows import (
     MXFP8Rows,
     SCALE_BLOCK,
     UNIT_SCALE,
-    empty_mxfp8_rows_bases,
-    mxfp8_rows_from_bases,
     pack_mxfp8_scales_for_dense_gemm,
 )
 
@@ -90,10 +88,15 @@ def _forward(source_2d: torch.Tensor, weight_values: torch.Tensor, weight_scale_
              stream_int: int | None) -> torch.Tensor:
     tokens = int(source_2d.shape[0])
     output_dtype_name(source_2d.dtype, _OWNER)
-    x_q = mxfp8_rows_from_bases(
-        *empty_mxfp8_rows_bases(tokens, padded_in, num_groups=1, device=source_2d.device),
-        tokens, padded_in, num_groups=1)
-    out = torch.empty((tokens, out_features, 1), dtype=source_2d.dtype, device=source_2d.device)
+    # The quantizer writes every byte of the scale atoms, padding included, so nothing is filled
+    # beforehand, and the GEMM reads no row-major scale bytes, so none are made.
+    device = source_2d.device
+    x_q = MXFP8Rows(
+        values=torch.empty((tokens, padded_in), dtype=torch.float8_e4m3fn, device=device),
+        scale_rows=None,
+        scale_mma=torch.empty((-(-tokens // 128) * (padded_in // K_STEP), 512), dtype=torch.uint8,
+                              device=device))
+    out = torch.empty((tokens, out_features, 1), dtype=source_2d.dtype, device=device)
     return quantize_then_gemm(pad_columns(source_2d, padded_in), weight_values, weight_scale_mma,
                               padded_k=padded_in, out_features=out_features, x_q=x_q, out=out,
                               bias=bias, stream=stream_int)
@@ -148,7 +151,14 @@ def mxfp8_linear(source: torch.Tensor, packed_weight: MXFP8LinearWeight, *,
     if rows.tokens == 0:
         output = rows.rows.new_empty((0, n))
         return rows.restore(output + bias if bias is not None else output, n)
-    if bias_fuses(bias, rows.rows.dtype, n):
+    fused = bias_fuses(bias, rows.rows.dtype, n)
+    if plain_eager(rows.rows, weight.values, weight.scale_mma, bias):
+        # What the custom ops below do, without the dispatcher round trip (most of a decode call).
+        output = _forward(rows.rows, weight.values, weight.scale_mma,
+                          padded_in=packed_weight.padded_in_features, out_features=n,
+                          bias=bias if fused else None, stream_int=cuda_stream_to_int(stream))
+        return rows.restore(output if fused or bias is None else output + bias, n)
+    if fused:
         output = torch.ops.b12x.mxfp8_linear_bias_fused(
             rows.rows, weight.values, weight.scale_mma, bias, packed_weight.padded_in_features, n,
             cuda_stream_to_int(stream))

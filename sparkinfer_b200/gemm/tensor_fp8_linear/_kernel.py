@@ -114,7 +114,8 @@ def _forward(source_2d: torch.Tensor, weight_values: torch.Tensor, weight_scale_
              output_scale: torch.Tensor, *, padded_in: int, out_features: int,
              out_dtype: torch.dtype, bias: torch.Tensor | None, stream_int: int | None) -> torch.Tensor:
     tokens = int(source_2d.shape[0])
-    codes = pad_columns(source_2d.view(torch.uint8), padded_in)
+    codes = (source_2d if source_2d.shape[1] == padded_in and source_2d.is_contiguous()
+             else pad_columns(source_2d.view(torch.uint8), padded_in))
     out = torch.empty((tokens, out_features), dtype=out_dtype, device=source_2d.device)
     del weight_scale_mma  # plain FP8: every block scale is 1.0 whatever the weight carries
     device = source_2d.device
@@ -122,8 +123,8 @@ def _forward(source_2d: torch.Tensor, weight_values: torch.Tensor, weight_scale_
         # Decode shapes: the weight-streaming kernel, which is written for block scales, fed
         # with cached scales of exactly 1.0 on both sides.
         launch.gemm_blockscaled(
-            _native.KIND_MXFP8, codes, _cached_unit_atoms(tokens, padded_in, device).view(torch.uint8),
-            weight_values, _cached_unit_atoms(out_features, padded_in, device).view(torch.uint8), out,
+            _native.KIND_MXFP8, codes, _cached_unit_atoms(tokens, padded_in, device),
+            weight_values, _cached_unit_atoms(out_features, padded_in, device), out,
             output_scale, tokens, out_features, padded_in, stream_int=stream_int, bias=bias)
     else:
         # Everything else: the unscaled E4M3 MMA, no scale bytes at all.
@@ -201,7 +202,15 @@ def tensor_fp8_linear(source: torch.Tensor, packed_weight: TensorFP8LinearWeight
                              f"got shape={tuple(bias.shape)}, dtype={bias.dtype}")
     if rows.tokens == 0:
         return rows.restore(torch.empty((0, n), dtype=out_dtype, device=rows.rows.device), n)
-    if bias_fuses(bias, out_dtype, n):
+    fused = bias_fuses(bias, out_dtype, n)
+    if launch.plain_eager(rows.rows, packed_weight.values, packed_weight.output_scale, bias):
+        # What the custom ops below do, without the dispatcher round trip.
+        output = _forward(rows.rows, packed_weight.values, packed_weight.scale_mma,
+                          packed_weight.output_scale, padded_in=packed_weight.padded_in_features,
+                          out_features=n, out_dtype=out_dtype, bias=bias if fused else None,
+                          stream_int=cuda_stream_to_int(stream))
+        return rows.restore(output if fused or bias is None else output + bias, n)
+    if fused:
         output = torch.ops.b12x.tensor_fp8_linear_bias_fused(
             rows.rows, packed_weight.values, packed_weight.scale_mma, packed_weight.output_scale,
             bias, packed_weight.padded_in_features, n, cuda_stream_to_int(stream))

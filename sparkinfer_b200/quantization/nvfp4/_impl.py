@@ -27,26 +27,21 @@ def _validate_shape(m: int, k: int) -> None:
 
 
 def _validate_launch_tensor(tensor: torch.Tensor, *, name: str, dtype: torch.dtype,
-                            shape: tuple[int, ...], device: torch.device) -> None:
+                            shape: tuple[int, ...], index: int) -> int:
+    """Address of the tensor's first byte, after the checks every operand has to pass."""
     if tensor.dtype != dtype:
         raise ValueError(f"{name} must have dtype {dtype}, got {tensor.dtype}")
-    if tuple(tensor.shape) != shape:
+    if tensor.shape != shape:
         raise ValueError(f"{name} must have shape {shape}, got {tuple(tensor.shape)}")
-    if tensor.device != device or tensor.device.type != "cuda":
-        raise ValueError(f"{name} must be on {device}, got {tensor.device}")
+    if not tensor.is_cuda or tensor.get_device() != index:
+        raise ValueError(f"{name} must be on cuda:{max(index, 0)}, got {tensor.device}")
     if not tensor.is_contiguous():
         raise ValueError(f"{name} must be contiguous")
+    return tensor.data_ptr()
 
 
-def _byte_interval(tensor: torch.Tensor) -> tuple[int, int]:
-    begin = tensor.untyped_storage().data_ptr() + tensor.storage_offset() * tensor.element_size()
-    return begin, begin + tensor.numel() * tensor.element_size()
-
-
-def _overlaps(lhs: torch.Tensor, rhs: torch.Tensor) -> bool:
-    a0, a1 = _byte_interval(lhs)
-    b0, b1 = _byte_interval(rhs)
-    return a0 < b1 and b0 < a1
+def _overlaps(a0: int, a_bytes: int, b0: int, b_bytes: int) -> bool:
+    return a0 < b0 + b_bytes and b0 < a0 + a_bytes
 
 
 def scale_storage_numel(m: int, k: int) -> int:
@@ -96,22 +91,24 @@ def compile_bf16_to_fp4_tma(m: int, k: int) -> Callable[..., None]:
     """
     _validate_shape(m, k)
     scale_numel = scale_storage_numel(m, k)
+    packed_numel = m * k // 2
 
     def launch(bf16_input, global_scale, packed_a_flat, scale_flat):
-        device = bf16_input.device
-        _validate_launch_tensor(bf16_input, name="bf16_input", dtype=torch.bfloat16,
-                                shape=(m, k), device=device)
-        _validate_launch_tensor(global_scale, name="global_scale", dtype=torch.float32,
-                                shape=(1,), device=device)
-        _validate_launch_tensor(packed_a_flat, name="packed_a_flat", dtype=torch.uint8,
-                                shape=(m * k // 2,), device=device)
-        _validate_launch_tensor(scale_flat, name="scale_flat", dtype=torch.uint8,
-                                shape=(scale_numel,), device=device)
-        if _overlaps(packed_a_flat, scale_flat):
+        index = bf16_input.get_device()
+        x = _validate_launch_tensor(bf16_input, name="bf16_input", dtype=torch.bfloat16,
+                                    shape=(m, k), index=index)
+        gs = _validate_launch_tensor(global_scale, name="global_scale", dtype=torch.float32,
+                                     shape=(1,), index=index)
+        codes = _validate_launch_tensor(packed_a_flat, name="packed_a_flat", dtype=torch.uint8,
+                                        shape=(packed_numel,), index=index)
+        scales = _validate_launch_tensor(scale_flat, name="scale_flat", dtype=torch.uint8,
+                                         shape=(scale_numel,), index=index)
+        if _overlaps(codes, packed_numel, scales, scale_numel):
             raise ValueError("packed_a_flat and scale_flat must not overlap")
-        if _overlaps(bf16_input, packed_a_flat) or _overlaps(bf16_input, scale_flat):
+        if (_overlaps(x, 4 * packed_numel, codes, packed_numel)
+                or _overlaps(x, 4 * packed_numel, scales, scale_numel)):
             raise ValueError("bf16_input must not overlap either output")
-        if _overlaps(global_scale, packed_a_flat) or _overlaps(global_scale, scale_flat):
+        if _overlaps(gs, 4, codes, packed_numel) or _overlaps(gs, 4, scales, scale_numel):
             raise ValueError("global_scale must not overlap either output")
         _launch.quantize_nvfp4_rows(bf16_input, global_scale, packed_a_flat, scale_flat)
 
