@@ -185,6 +185,19 @@ int b12x_b200_gemm_blockscaled_smallm_grouped(int kind, const void* x, const voi
                                               int* status, b12x_b200_stream_t stream);
 
 /*
+ * The GEMM of a linear layer whose packed weight rows are longer than K: MXFP8 or unscaled FP8
+ * operands, x [M, K] dense, w [N, ldw] with ldw >= K bytes between rows (a multiple of 16) of which
+ * the first K are multiplied. K % 32 == 0; scale atoms cover ceil(K / 128) atoms per row tile, as
+ * everywhere. decode != 0 runs the weight-streaming kernel (1 <= M <= 128, MXFP8), else the tiled
+ * kernels. Workspace as b12x_b200_gemm_grouped_workspace_bytes(kind, decode, m, n, k, 1, 0, 0).
+ */
+int b12x_b200_gemm_linear(int kind, int decode, const void* x, const void* sf_x, const void* w,
+                          int64_t ldw, const void* sf_w, void* c, int c_dtype, const float* alpha,
+                          int64_t m, int64_t n, int64_t k, int64_t ldc, void* workspace,
+                          int64_t workspace_bytes, const b12x_b200_epilogue_t* epilogue,
+                          int* status, b12x_b200_stream_t stream);
+
+/*
  * Decode-shape (1 <= M <= 128) variant of b12x_b200_gemm_blockscaled: the weight matrix is
  * streamed once, split evenly over all SMs along N and K (stream-K), and partial sums meet in
  * a caller-owned FP32 workspace. Stands in for the reference's small-M split-K policy and its

@@ -294,12 +294,16 @@ def gemm_blockscaled(kind: int, a: torch.Tensor, sfa: torch.Tensor | None, b: to
                      m: int, n: int, k: int, *, ldc: int | None = None, block_n: int = 0,
                      sm_count: int = 0, stream_int: int | None = None,
                      small_m: bool | None = None, bias: torch.Tensor | None = None,
-                     quantized_c: QuantizedC | None = None, groups: int = 1) -> None:
+                     quantized_c: QuantizedC | None = None, groups: int = 1,
+                     ldb: int | None = None) -> None:
     """``c[M, ldc] = cvt(alpha * (a . sfa)(b . sfb)^T)``. ``a``/``b`` are row pointers to K-major
     code matrices, ``sfa``/``sfb`` point at the first scale atom. With ``groups > 1`` the
     tensors hold that many problems of the same shape group after group (operands ``[L, rows,
     K]``, each group's dense scale atoms, outputs ``[L, M, ldc]``) and all of them run in one
     launch.
+
+    ``ldb``: bytes between the rows of an MXFP8 / FP8 ``b`` that is wider than K (one group, no
+    forced tile).
 
     Decode shapes (see :func:`route_to_decode_kernel`; never when a tile width is forced, always
     with ``small_m=True``) go to the weight-streaming stream-K kernel, everything else to the
@@ -335,7 +339,11 @@ def gemm_blockscaled(kind: int, a: torch.Tensor, sfa: torch.Tensor | None, b: to
             None if plain else sfb.data_ptr(), c.data_ptr(), dtype_code,
             alpha.data_ptr() if alpha is not None else None,
             m, n, k, ldc if ldc is not None else n, groups)
-    if decode:
+    if ldb is not None and ldb != k:
+        rc = _call_on(index, lib.b12x_b200_gemm_linear, kind, 1 if decode else 0, *head[1:4], ldb,
+                      *head[4:12], work_ptr, work_bytes, ep_ref, _status_of(index).data_ptr(),
+                      stream)
+    elif decode:
         rc = _call_on(index, lib.b12x_b200_gemm_blockscaled_smallm_grouped, *head, work_ptr,
                       work_bytes, ep_ref, sm_count, _status_of(index).data_ptr(), stream)
     else:

@@ -52,6 +52,15 @@ def pad_columns(rows: torch.Tensor, width: int) -> torch.Tensor:
     return torch.nn.functional.pad(rows, (0, width - have))
 
 
+def multipliable_rows(rows: torch.Tensor, width: int) -> torch.Tensor:
+    """``rows [T, K]`` for a weight padded to ``width`` columns. The kernels read K columns and
+    take the weight's longer rows as a pitch, so nothing is padded here, unless the rows do not
+    start where their 16-byte loads can: the padded copy does."""
+    if rows.shape[1] != width and rows.data_ptr() % 16 != 0:
+        return pad_columns(rows, width)
+    return rows.contiguous()
+
+
 @dataclass(frozen=True)
 class SourceRows:
     """A linear's input seen as ``[tokens, K]`` rows."""
@@ -143,12 +152,12 @@ def bias_fuses(bias: torch.Tensor | None, out_dtype: torch.dtype, out_features: 
 
 def mxfp8_gemm(x_q: MXFP8Rows, weight_values: torch.Tensor, weight_scale_mma: torch.Tensor, *,
                tokens: int, k: int, out_features: int, out: torch.Tensor,
-               bias: torch.Tensor | None, stream: object) -> None:
+               bias: torch.Tensor | None, stream: object, ldb: int | None = None) -> None:
     """``out [T, N, 1] = x_q @ W^T (+ bias)`` on MXFP8 rows, straight through the launcher."""
     launch.gemm_blockscaled(
         _native.KIND_MXFP8, x_q.values, x_q.scale_mma, weight_values, weight_scale_mma, out, None,
         tokens, out_features, k, ldc=out.stride(0) if tokens > 1 else out_features,
-        stream_int=cuda_stream_to_int(stream), bias=bias)
+        stream_int=cuda_stream_to_int(stream), bias=bias, ldb=ldb)
 
 
 def quantize_then_gemm(rows: torch.Tensor, weight_values: torch.Tensor,
@@ -156,20 +165,22 @@ def quantize_then_gemm(rows: torch.Tensor, weight_values: torch.Tensor,
                        x_q: MXFP8Rows, out: torch.Tensor, bias: torch.Tensor | None,
                        stream: object, bias_in_place: bool = False) -> torch.Tensor:
     """The forward step of the MXFP8-based linears on caller-provided buffers: row-quantize
-    ``rows [T, padded_k]`` into ``x_q``, multiply into ``out [T, N, 1]``. Returns ``out[:, :, 0]``
+    ``rows [T, K]`` (K up to the weight's ``padded_k``) into ``x_q``, multiply into ``out [T, N, 1]``. Returns ``out[:, :, 0]``
     with the bias applied: in the GEMM epilogue when :func:`bias_fuses`, else by torch (into
     ``out`` itself with ``bias_in_place``, as a bound call must, or as a new tensor)."""
     tokens = int(rows.shape[0])
     quantize_mxfp8_rows(rows, x_q.values, x_q.scale_rows, x_q.scale_mma, stream=stream)
     fused = bias_fuses(bias, out.dtype, out_features)
-    mxfp8_gemm(x_q, weight_values, weight_scale_mma, tokens=tokens, k=padded_k,
-               out_features=out_features, out=out, bias=bias if fused else None, stream=stream)
+    mxfp8_gemm(x_q, weight_values, weight_scale_mma, tokens=tokens, k=int(rows.shape[1]),
+               out_features=out_features, out=out, bias=bias if fused else None, stream=stream,
+               ldb=padded_k)
     result = out.select(2, 0)
     if bias is not None and not fused:
         result = result.add_(bias) if bias_in_place else result + bias
     return result
 
 
-__all__ = ["ActivationPlan", "K_STEP", "LINEAR_DTYPES", "SourceRows", "bias_fuses", "mxfp8_gemm",
+__all__ = ["ActivationPlan", "K_STEP", "LINEAR_DTYPES", "SourceRows", "bias_fuses",
+           "multipliable_rows", "mxfp8_gemm",
            "output_dtype_name", "pad_columns", "quantize_then_gemm", "require_cuda_tensor",
            "round_up"]

@@ -70,6 +70,12 @@ SIGNATURES = {
          _c_i64, _c_i64, _c_i64, _c_i64, _c_i64, _c_void_p, _c_i64, _c_epilogue_p, _c_int,
          _c_void_p, _c_void_p],
     ),
+    "b12x_b200_gemm_linear": (
+        _c_int,
+        [_c_int, _c_int, _c_void_p, _c_void_p, _c_void_p, _c_i64, _c_void_p, _c_void_p, _c_int,
+         _c_void_p, _c_i64, _c_i64, _c_i64, _c_i64, _c_void_p, _c_i64, _c_epilogue_p, _c_void_p,
+         _c_void_p],
+    ),
     "b12x_b200_gemm_blockscaled_smallm_ex": (
         _c_int,
         [_c_int, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_void_p,

@@ -198,7 +198,7 @@ int gemm_blockscaled_impl(int kind, const void* a, const void* sfa, const void* 
                           int64_t ldc, int64_t groups, int block_n, int sm_count, void* workspace,
                           int64_t workspace_bytes, const b12x_b200_epilogue_t* epilogue,
                           int* status, b12x_b200_stream_t stream,
-                          const ScatterPlan* scatter = nullptr) {
+                          const ScatterPlan* scatter = nullptr, int64_t ldb = 0) {
   if (groups < 1 || groups > 65535)
     return fail(B12X_B200_ERR_INVALID_ARGUMENT, "groups must be in [1, 65535]");
   if (kind != B12X_B200_KIND_MXFP8 && kind != B12X_B200_KIND_NVFP4 && kind != B12X_B200_KIND_FP8 &&
@@ -265,7 +265,7 @@ int gemm_blockscaled_impl(int kind, const void* a, const void* sfa, const void* 
   rc = make_operand_map(&map_a, a, uint64_t(m), uint64_t(row_bytes), 128, uint64_t(groups));
   if (rc != B12X_B200_OK) return rc;
   rc = make_operand_map(&map_b, b, uint64_t(n), uint64_t(row_bytes),
-                        use_pair ? 128u : uint32_t(bn), uint64_t(groups));
+                        use_pair ? 128u : uint32_t(bn), uint64_t(groups), uint64_t(ldb));
   if (rc != B12X_B200_OK) return rc;
 
   GemmParams p;
@@ -642,6 +642,7 @@ struct SmallMCall {
   cudaStream_t stream;
   const b12x_b200_epilogue_t* epilogue = nullptr;
   int64_t groups = 1;
+  int64_t ldw = 0;             // bytes between weight rows (0: dense rows)
   int64_t x_group_stride = 0;  // fused rows: elements between groups (0: group-major rows)
   // Inverse rotary embedding in front of the fused MXFP8 quantizer (null positions: none).
   const void* rope_positions = nullptr;
@@ -720,7 +721,8 @@ int run_smallm(const SmallMCall& a, const SmallMPlan& pl, void* workspace,
     return fail(B12X_B200_ERR_INVALID_ARGUMENT, "workspace smaller than b12x_b200_gemm_smallm_workspace_bytes");
   const int64_t row_bytes = (a.kind == B12X_B200_KIND_MXFP8) ? a.k : a.k / 2;
   CUtensorMap map_w, map_x;
-  int rc = make_operand_map(&map_w, a.w, uint64_t(a.n), uint64_t(row_bytes), 128, uint64_t(a.groups));
+  int rc = make_operand_map(&map_w, a.w, uint64_t(a.n), uint64_t(row_bytes), 128,
+                            uint64_t(a.groups), uint64_t(a.ldw));
   if (rc != B12X_B200_OK) return rc;
   if (fused) {
     const uint32_t elems = (a.kind == B12X_B200_KIND_MXFP8) ? 128u : 256u;
@@ -858,6 +860,27 @@ extern "C" int b12x_b200_gemm_blockscaled_smallm_grouped(
                   reinterpret_cast<cudaStream_t>(stream)};
   a.epilogue = epilogue;
   a.groups = groups;
+  return smallm_entry(a, workspace, workspace_bytes);
+}
+
+extern "C" int b12x_b200_gemm_linear(int kind, int decode, const void* x, const void* sf_x,
+                                     const void* w, int64_t ldw, const void* sf_w, void* c,
+                                     int c_dtype, const float* alpha, int64_t m, int64_t n,
+                                     int64_t k, int64_t ldc, void* workspace,
+                                     int64_t workspace_bytes, const b12x_b200_epilogue_t* epilogue,
+                                     int* status, b12x_b200_stream_t stream) {
+  if (kind != B12X_B200_KIND_MXFP8 && kind != B12X_B200_KIND_FP8)
+    return fail(B12X_B200_ERR_INVALID_ARGUMENT, "a linear's operands are MXFP8 or FP8");
+  if (ldw < k || ldw % 16 != 0)
+    return fail(B12X_B200_ERR_ALIGNMENT, "weight rows must be 16-byte multiples of at least K bytes");
+  if (!decode)
+    return gemm_blockscaled_impl(kind, x, sf_x, w, sf_w, c, c_dtype, alpha, m, n, k, ldc, 1, 0, 0,
+                                 workspace, workspace_bytes, epilogue, status, stream, nullptr, ldw);
+  SmallMCall a = {kind, x,     sf_x, nullptr, 0,   nullptr,  w,      sf_w,    c, c_dtype,
+                  alpha, m,    n,    k,       ldc, 0, status, nullptr,
+                  reinterpret_cast<cudaStream_t>(stream)};
+  a.epilogue = epilogue;
+  a.ldw = ldw;
   return smallm_entry(a, workspace, workspace_bytes);
 }
 

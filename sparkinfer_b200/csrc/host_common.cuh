@@ -99,13 +99,15 @@ inline int make_operand_map_2d(CUtensorMap* map, const void* base, uint64_t rows
 
 // Stack of `groups` K-major byte matrices [groups, rows, row_bytes] -> boxes of 128 bytes x
 // box_rows x 1 group, 128-byte swizzle. A box never crosses into the next group: rows at or
-// beyond `rows` are out of bounds and read as zeros.
+// beyond `rows` are out of bounds and read as zeros. `pitch`: bytes between rows (0: row_bytes),
+// for one group only; bytes of a row at or beyond row_bytes read as zeros too.
 inline int make_operand_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes,
-                     uint32_t box_rows, uint64_t groups = 1) {
+                     uint32_t box_rows, uint64_t groups = 1, uint64_t pitch = 0) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return fail(B12X_B200_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
   const cuuint64_t dims[3] = {row_bytes, rows, groups};
-  const cuuint64_t strides[2] = {row_bytes, rows * row_bytes};
+  if (pitch == 0) pitch = row_bytes;
+  const cuuint64_t strides[2] = {pitch, rows * pitch};
   const cuuint32_t box[3] = {128, box_rows, 1};
   const cuuint32_t elem_strides[3] = {1, 1, 1};
   const CUresult r =

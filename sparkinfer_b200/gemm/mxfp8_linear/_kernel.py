@@ -14,6 +14,7 @@ from ..._lib.linear_core import (
     K_STEP,
     SourceRows,
     bias_fuses,
+    multipliable_rows,
     output_dtype_name,
     pad_columns,
     quantize_then_gemm,
@@ -91,13 +92,14 @@ def _forward(source_2d: torch.Tensor, weight_values: torch.Tensor, weight_scale_
     # The quantizer writes every byte of the scale atoms, padding included, so nothing is filled
     # beforehand, and the GEMM reads no row-major scale bytes, so none are made.
     device = source_2d.device
+    rows = multipliable_rows(source_2d, padded_in)
     x_q = MXFP8Rows(
-        values=torch.empty((tokens, padded_in), dtype=torch.float8_e4m3fn, device=device),
+        values=torch.empty(rows.shape, dtype=torch.float8_e4m3fn, device=device),
         scale_rows=None,
         scale_mma=torch.empty((-(-tokens // 128) * (padded_in // K_STEP), 512), dtype=torch.uint8,
                               device=device))
     out = torch.empty((tokens, out_features, 1), dtype=source_2d.dtype, device=device)
-    return quantize_then_gemm(pad_columns(source_2d, padded_in), weight_values, weight_scale_mma,
+    return quantize_then_gemm(rows, weight_values, weight_scale_mma,
                               padded_k=padded_in, out_features=out_features, x_q=x_q, out=out,
                               bias=bias, stream=stream_int)
 

@@ -22,6 +22,7 @@ from ..._lib.linear_core import (
     LINEAR_DTYPES,
     SourceRows,
     bias_fuses,
+    multipliable_rows,
     pad_columns,
     require_cuda_tensor,
     round_up,
@@ -114,8 +115,8 @@ def _forward(source_2d: torch.Tensor, weight_values: torch.Tensor, weight_scale_
              output_scale: torch.Tensor, *, padded_in: int, out_features: int,
              out_dtype: torch.dtype, bias: torch.Tensor | None, stream_int: int | None) -> torch.Tensor:
     tokens = int(source_2d.shape[0])
-    codes = (source_2d if source_2d.shape[1] == padded_in and source_2d.is_contiguous()
-             else pad_columns(source_2d.view(torch.uint8), padded_in))
+    codes = multipliable_rows(source_2d.view(torch.uint8), padded_in)
+    k = int(codes.shape[1])
     out = torch.empty((tokens, out_features), dtype=out_dtype, device=source_2d.device)
     del weight_scale_mma  # plain FP8: every block scale is 1.0 whatever the weight carries
     device = source_2d.device
@@ -125,12 +126,12 @@ def _forward(source_2d: torch.Tensor, weight_values: torch.Tensor, weight_scale_
         launch.gemm_blockscaled(
             _native.KIND_MXFP8, codes, _cached_unit_atoms(tokens, padded_in, device),
             weight_values, _cached_unit_atoms(out_features, padded_in, device), out,
-            output_scale, tokens, out_features, padded_in, stream_int=stream_int, bias=bias)
+            output_scale, tokens, out_features, k, stream_int=stream_int, bias=bias, ldb=padded_in)
     else:
         # Everything else: the unscaled E4M3 MMA, no scale bytes at all.
         launch.gemm_blockscaled(_native.KIND_FP8, codes, None, weight_values, None, out,
-                                output_scale, tokens, out_features, padded_in,
-                                stream_int=stream_int, bias=bias)
+                                output_scale, tokens, out_features, k, stream_int=stream_int,
+                                bias=bias, ldb=padded_in)
     return out
 
 
