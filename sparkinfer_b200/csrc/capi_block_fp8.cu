@@ -3,6 +3,7 @@
 #include "host_common.cuh"
 
 #include "gemm_block_fp8.cuh"
+#include "gemm_block_fp8_pair.cuh"
 #include "gemm_block_fp8_smallm.cuh"
 
 using namespace b12x_b200;
@@ -148,6 +149,58 @@ int run_block_fp8_small(const BlockFp8SmallPlan& pl, const void* a, const float*
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// Tiled kernels
+// ------------------------------------------------------------------------------------------
+template <bool BIAS>
+int launch_block_fp8_pair(const CUtensorMap& map_a, const CUtensorMap& map_b,
+                          const CUtensorMap& map_c, const BlockFp8Params& p, int pairs,
+                          cudaStream_t stream) {
+  using T = BlockFp8PairTile;
+  static std::atomic<bool> set_for[64];  // zero-initialised; setting the attribute twice is harmless
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && !set_for[dev]) {
+    const cudaError_t err =
+        cudaFuncSetAttribute(gemm_block_fp8_pair_kernel<BIAS>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmemBytes);
+    if (err != cudaSuccess) return fail_cuda(err, "cudaFuncSetAttribute");
+    set_for[dev] = true;
+  }
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
+  cfg.blockDim = dim3(T::kThreads, 1, 1);
+  cfg.dynamicSmemBytes = T::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t err =
+      cudaLaunchKernelEx(&cfg, gemm_block_fp8_pair_kernel<BIAS>, map_a, map_b, map_c, p);
+  if (err != cudaSuccess) return fail_cuda(err, "gemm_block_fp8_pair launch");
+  return B12X_B200_OK;
+}
+
+// The CTA-pair kernel is faster per round of tiles but has more to do between two tiles. Single-CTA
+// against pair kernel in us: K = 512 100 / 109 (8192 x 16384) and 10.3 / 12.5 (1024 x 4096), K = 1536
+// 14.5 / 16.6 (700 x 5120), K = 2048 16.6 / 17.4 (200 x 14336) but 138 / 132 (8192 x 7168), K = 4096 162 / 145
+// (8192 x 4096), K = 7168 39.0 / 37.1 (256 x 7168) and 535 / 499 (4096 x 18432), K = 16384 84 / 77
+// (2048 x 2048): the line is drawn at K = 3072. An odd number of 128-row tiles costs it a row of
+// tiles, so it must not need more rounds (640 x 7168: 84 pair tiles are two rounds of 74 pairs,
+// 140 single tiles are one of 148 SMs).
+bool block_fp8_pair_wins(int64_t m, int64_t n, int64_t k, int sms) {
+  if (m <= 128 || k < 3072 || sms < 2) return false;
+  const int64_t tiles_n = (n + 255) / 256, pairs = sms / 2;
+  const int64_t pair_rounds = ((m + 255) / 256 * tiles_n + pairs - 1) / pairs;
+  const int64_t single_rounds = ((m + 127) / 128 * tiles_n + sms - 1) / sms;
+  return pair_rounds <= single_rounds;
+}
+
 int gemm_block_fp8_impl(const void* a, const float* sfa, const void* b, const float* sfb, void* c,
                         int c_dtype, const float* alpha, int64_t m, int64_t n, int64_t k,
                         int64_t ldc, int sm_count, const b12x_b200_epilogue_t* epilogue,
@@ -180,10 +233,14 @@ int gemm_block_fp8_impl(const void* a, const float* sfa, const void* b, const fl
                                epilogue ? epilogue->bias : nullptr, status,
                                reinterpret_cast<cudaStream_t>(stream));
 
+  const int64_t pair_tiles = ((m + 255) / 256) * ((n + 255) / 256);
+  const bool use_pair = block_fp8_pair_wins(m, n, k, sms);
+
   CUtensorMap map_a, map_b;
   rc = make_operand_map_2d(&map_a, a, uint64_t(m), uint64_t(k), BlockFp8Tile::BM);
   if (rc != B12X_B200_OK) return rc;
-  rc = make_operand_map_2d(&map_b, b, uint64_t(n), uint64_t(k), BlockFp8Tile::BN);
+  rc = make_operand_map_2d(&map_b, b, uint64_t(n), uint64_t(k),
+                           use_pair ? BlockFp8PairTile::kHalf / 2 : BlockFp8Tile::BN);
   if (rc != B12X_B200_OK) return rc;
 
   BlockFp8Params p;
@@ -228,6 +285,14 @@ int gemm_block_fp8_impl(const void* a, const float* sfa, const void* b, const fl
     rc = make_output_map_2d(&map_c, c, uint64_t(m), uint64_t(n), uint64_t(ldc));
     if (rc != B12X_B200_OK) return rc;
     p.use_tma_store = 1;
+  }
+  if (use_pair) {
+    p.tiles_m = int((m + 255) / 256);
+    p.group_m = 16;
+    const int pairs = int(pair_tiles < sms / 2 ? pair_tiles : sms / 2);
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    return p.bias ? launch_block_fp8_pair<true>(map_a, map_b, map_c, p, pairs, s)
+                  : launch_block_fp8_pair<false>(map_a, map_b, map_c, p, pairs, s);
   }
   if (p.bias)
     gemm_block_fp8_kernel<true><<<grid, BlockFp8Tile::kThreads, BlockFp8Tile::kSmemBytes,

@@ -435,6 +435,15 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t cluster_addr) {
                : "memory");
 }
 
+// The same with one arrival in each CTA of the pair, on the mbarrier at `smem_addr`'s offset.
+__device__ __forceinline__ void tc_commit_pair_both(uint32_t smem_addr) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
+      "[%0], %1;"
+      ::"r"(smem_addr), "h"(static_cast<uint16_t>(3))
+      : "memory");
+}
+
 // Scale atom copy executed in both CTAs of the pair: each reads its own shared memory at the
 // descriptor's offset and writes its own tensor memory.
 __device__ __forceinline__ void tc_copy_sf_atom_pair(uint32_t taddr, uint64_t sdesc) {

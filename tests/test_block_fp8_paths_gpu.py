@@ -56,3 +56,26 @@ def test_few_rows(m, n, k):
     (100, torch.float16, {"alpha": 0.125}), (100, torch.bfloat16, {"bias": True, "ldc": 1153})])
 def test_few_rows_epilogues(m, dtype, kwargs):
     _check(m, 1152, 1152, dtype, **kwargs)
+
+
+# CTA-pair kernel (M > 128, K >= 3072, no more rounds than the single-CTA kernel): a last row tile
+# of one row, of one CTA of the pair and full; N with half a column tile; scale batches of eight
+# k-blocks with and without a remainder; more than one tile per pair.
+@pytest.mark.parametrize("m,n,k", [(129, 256, 3072), (257, 128, 3200), (384, 384, 3968),
+                                   (512, 1152, 4096), (1100, 9600, 3072), (2304, 4352, 3328)])
+def test_pair_tiles(m, n, k):
+    _check(m, n, k, torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype,kwargs", [
+    (torch.float32, {}), (torch.float32, {"bias": True}), (torch.float16, {"bias": True}),
+    (torch.bfloat16, {"ldc": 1160}), (torch.bfloat16, {"ldc": 1157, "bias": True}),
+    (torch.float16, {"alpha": 0.125})])
+def test_pair_epilogues(dtype, kwargs):
+    _check(390, 1152, 3200, dtype, **kwargs)
+
+
+# Neighbours of the rule's lines run the single-CTA kernel.
+@pytest.mark.parametrize("m,n,k", [(129, 256, 2944), (640, 7168, 3072)])
+def test_beside_the_pair_rule(m, n, k):
+    _check(m, n, k, torch.bfloat16)
