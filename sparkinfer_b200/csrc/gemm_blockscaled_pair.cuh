@@ -10,9 +10,9 @@
 //
 // Hand-shake per stage s (all waits bounded):
 //   producer (each CTA)  : wait own empty[s] -> arm own full[s], issue own loads
-//   relay (peer, warp 1) : wait own full[s]  -> arrive on the leader's peer_full[s]
-//   issuer (leader, w 1) : wait own full[s] and peer_full[s] -> scale copies + 4 MMAs for the
-//                          pair -> tcgen05.commit to empty[s] of both CTAs (two commits)
+//   relay (peer, warp 1) : wait own full[s]  -> arrive on the leader's full[s]
+//   issuer (leader, w 1) : wait own full[s] -> scale copies + 4 MMAs for the pair -> one
+//                          tcgen05.commit to empty[s] of both CTAs
 //   epilogue (each CTA)  : wait own acc_full (committed by the leader to both CTAs) -> pull own
 //                          128 x 256 accumulator into registers -> arrive on the leader's
 //                          acc_empty -> convert, stage in swizzled shared memory, TMA store
@@ -184,8 +184,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* c_stage = smem + T::kStages * T::kStageBytes;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(c_stage + T::kCStageBytes);
-  uint64_t* peer_full_bar = full_bar + T::kStages;   // used in the leader only
-  uint64_t* empty_bar = peer_full_bar + T::kStages;
+  uint64_t* empty_bar = full_bar + T::kStages;
   uint64_t* acc_full_bar = empty_bar + T::kStages;
   uint64_t* acc_empty_bar = acc_full_bar + 2;        // used in the leader only
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty_bar + 2);
@@ -198,8 +197,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < T::kStages; ++s) {
-      mbar_init(&full_bar[s], T::kScaled ? 2 : 1);  // operand producer (+ scale producer)
-      mbar_init(&peer_full_bar[s], 1);
+      // Operand producer (+ scale producer); in the leader also the peer's full stage, relayed.
+      mbar_init(&full_bar[s], (T::kScaled ? 2 : 1) + (leader ? 1 : 0));
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -332,7 +331,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           break;
         }
         if (elect_one())
-          mbar_arrive_cluster(map_to_cta(smem_addr_u32(&peer_full_bar[stage]), 0));
+          mbar_arrive_cluster(map_to_cta(smem_addr_u32(&full_bar[stage]), 0));
         __syncwarp();
         if (++stage == T::kStages) { stage = 0; phase ^= 1; }
       }
@@ -358,9 +357,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       tc_fence_after_sync();
       const uint32_t d_taddr = acc * BN;
       for (int kt = w.kt_begin; kt < w.kt_end; ++kt) {
-        const bool got_local = mbar_wait_bounded(&full_bar[stage], phase, abort_flag);
-        if (!got_local ||
-            !mbar_wait_bounded_cluster(&peer_full_bar[stage], phase, abort_flag)) {
+        if (!mbar_wait_bounded_cluster(&full_bar[stage], phase, abort_flag)) {
           *abort_flag = 1;
           if (p.status && lane == 0) atomicMax(p.status, kStatusMmaTimeout);
           ok = false;
@@ -384,7 +381,9 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           }
           const uint64_t adesc = make_kmajor_sw128_desc(st);
           const uint64_t bdesc = make_kmajor_sw128_desc(st + T::kABytes);
-          for (int j = 0; j < mmas; ++j) {
+#pragma unroll
+          for (int j = 0; j < T::kMmasPerStage; ++j) {
+            if (j >= mmas) break;
             const uint32_t accumulate = (kt > w.kt_begin || j > 0) ? 1u : 0u;
             if constexpr (KIND == kFp8)
               tc_mma_f8_pair(d_taddr, adesc + 2 * j, bdesc + 2 * j, idesc_base, accumulate);
@@ -402,14 +401,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
                                T::kSfaCol0 + j * 4, T::kSfbCol0 + j * T::kSfbRowAtoms * 4);
           }
           // Free the stage in both CTAs; publish the accumulator to both after the last step.
-          const uint32_t empty_addr = smem_addr_u32(&empty_bar[stage]);
-          tc_commit_pair(empty_addr);
-          tc_commit_pair(map_to_cta(empty_addr, 1));
-          if (kt == w.kt_end - 1) {
-            const uint32_t full_addr = smem_addr_u32(&acc_full_bar[acc]);
-            tc_commit_pair(full_addr);
-            tc_commit_pair(map_to_cta(full_addr, 1));
-          }
+          tc_commit_pair_both(smem_addr_u32(&empty_bar[stage]));
+          if (kt == w.kt_end - 1) tc_commit_pair_both(smem_addr_u32(&acc_full_bar[acc]));
         }
         __syncwarp();
         if (++stage == T::kStages) { stage = 0; phase ^= 1; }
