@@ -496,7 +496,7 @@ namespace {
 
 struct SmallMPlan {
   int m_pad, tiles, tiles_per_group, k_tiles, k_atoms, grid, max_segments, stages, stage_bytes;
-  int issuers, sf_col0, tmem_cols, raw_rows;
+  int issuers, sf_col0, tmem_cols, raw_rows, whole_tiles;
   size_t partial_bytes, total_bytes;
 };
 
@@ -526,12 +526,31 @@ int plan_smallm(int kind, int64_t m, int64_t n, int64_t k, int sms, bool fused, 
   // partial sums at all; with more tiles than SMs one CTA per SM streams an equal share.
   // (One CTA per SM regardless, which splits every tile of a 112-tile problem over two or three
   // CTAs, was measured slower: 12.6 us against 10.9 us for 16 x 14336 x 4096.)
+  //
+  // Cutting tiles costs the exchange of partials (write, fence, count, the last arriver's loads
+  // behind its own weight requests) at the end of the kernel; keeping them whole costs the time in
+  // which only some SMs still stream. Both in KiB of weights, at the ~95 GB/s one SM streams:
+  // the exchange is worth `limit`, whole tiles cost what is left of a tile when the balanced split
+  // would be through with it. Measured, cut -> whole, us: 64 x 20000 x 1024 NVFP4 13.1 -> 7.5, 33 x 30000 x
+  // 2048 14.4 -> 9.3 (MXFP8 18.5 -> 14.6), 64 x 57344 x 4096 33.8 -> 27.9 (MXFP8 50.4 -> 48.7), 5 x 40000 x 512
+  // 8.3 -> 5.5, 16 x 47232 x 2560 16.1 -> 13.3, 4 x 32768 x 3072 13.4 -> 11.2; beyond the line 1 x 20000 x 4096
+  // MXFP8 18.2 -> 22.0, 16 x 24000 x 6144 29.4 -> 33.5, 16 x 57344 x 4096 43.7 -> 46.1, 8 x 28672 x 8192 42.1 -> 43.6.
+  const int64_t tile_kib = int64_t(pl.k_tiles) * 18;
+  const int64_t limit = pl.m_pad <= 16 ? 240 : pl.m_pad <= 32 ? 400 : 600;
   if (pl.tiles <= sms) {
     int per_tile = sms / pl.tiles;
     if (per_tile > pl.k_tiles) per_tile = pl.k_tiles;
+    // The last arriver adds one slot per CTA of the tile (0.2 us each for 16 rows, 0.6 for 32, 1.5
+    // for 64), a p-th of the tile takes 0.19 us * k_tiles / p: the sum is least at this p.
+    const int64_t slot_cost = pl.m_pad <= 16 ? 12 : pl.m_pad <= 32 ? 31 : 80;   // in tenths of 0.19 us
+    while (per_tile > 1 && int64_t(per_tile) * per_tile * slot_cost > int64_t(pl.k_tiles) * 10) --per_tile;
+    if (tile_kib * (per_tile - 1) < limit * per_tile) per_tile = 1;
     pl.grid = pl.tiles * per_tile;
+    pl.whole_tiles = per_tile == 1 ? 1 : 0;
   } else {
     pl.grid = int(units < sms ? units : sms);
+    const int left = pl.tiles % sms;   // tiles of the last round; about 100 SMs saturate HBM
+    pl.whole_tiles = (left == 0 || tile_kib * (100 - left) < limit * 100) ? 1 : 0;
   }
   const int64_t units_per_cta = units / pl.grid;  // >= 1
   int64_t seg = (pl.k_tiles + units_per_cta - 1) / units_per_cta + 1;
@@ -757,6 +776,7 @@ int run_smallm(const SmallMCall& a, const SmallMPlan& pl, void* workspace,
   p.c_group_elems = a.m * a.ldc;
   p.k_tiles = pl.k_tiles;
   p.k_atoms_total = pl.k_atoms;
+  p.whole_tiles = pl.whole_tiles;
   p.max_segments = pl.max_segments;
   p.num_stages = pl.stages;
   p.stage_bytes = pl.stage_bytes;

@@ -8,7 +8,9 @@
 //
 // Work is cut stream-K style. A unit is (weight tile of 128 rows, k-tile of 128 bytes of K);
 // units are numbered tile-major and CTA c of G takes units [c*U/G, (c+1)*U/G), i.e. every
-// CTA streams the same number of bytes (+-1 unit) whatever N is. A CTA range covers a run of
+// CTA streams the same number of bytes (+-1 unit) whatever N is; or, where the exchange of
+// partials would cost more than an uneven last round (whole_tiles, see the plan on the host), the
+// range ends are moved to tile boundaries. A CTA range covers a run of
 // segments, one per tile it touches. A segment that spans its whole tile is converted and
 // stored directly. Otherwise the FP32 partial goes to scratch slot (tile, segment index) and
 // a per-tile counter is bumped; the CTA that brings the counter to the segment count adds the
@@ -82,6 +84,7 @@ struct SmallMParams {
   long long sf_w_group_bytes, sf_x_group_bytes, c_group_elems;
   int k_tiles;             // ceil(K / elems per stage)
   int k_atoms_total;
+  int whole_tiles;         // CTA ranges end at tile boundaries (no partial sums)
   int max_segments;        // scratch slots per tile
   int num_stages;
   int stage_bytes;
@@ -407,8 +410,10 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w,
   // Unit arithmetic is 32-bit in the loops (the host rejects tiles * k_tiles >= 2^31); the
   // range ends use 64-bit products once.
   const int units = p.tiles * p.k_tiles;
-  const int u_begin = static_cast<int>(static_cast<long long>(units) * blockIdx.x / gridDim.x);
-  const int u_end = static_cast<int>(static_cast<long long>(units) * (blockIdx.x + 1) / gridDim.x);
+  const int grain = p.whole_tiles ? p.k_tiles : 1;   // units a range end is a multiple of
+  const long long grains = p.whole_tiles ? p.tiles : units;
+  const int u_begin = static_cast<int>(grains * blockIdx.x / gridDim.x) * grain;
+  const int u_end = static_cast<int>(grains * (blockIdx.x + 1) / gridDim.x) * grain;
   const uint32_t smem_u32 = smem_addr_u32(smem);
   const uint32_t x_bytes = static_cast<uint32_t>(p.m_pad) * 128u;
   // Bytes of raw BF16 rows one stage of the fused variant receives.
