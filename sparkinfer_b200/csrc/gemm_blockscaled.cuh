@@ -125,6 +125,28 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
   return r;
 }
 
+// vals = float(cvt(vals)) + bias for 32 columns of a 2-byte output type, bias packed in pairs.
+__device__ __forceinline__ void add_packed_bias_32(float (&vals)[32], const uint32_t (&packed)[16],
+                                                   int out_dtype) {
+  if (out_dtype == kOutBf16) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const uint32_t y = pack_bf16x2(vals[2 * i], vals[2 * i + 1]);
+      vals[2 * i] = __fadd_rn(__uint_as_float(y << 16), __uint_as_float(packed[i] << 16));
+      vals[2 * i + 1] = __fadd_rn(__uint_as_float(y & 0xFFFF0000u), __uint_as_float(packed[i] & 0xFFFF0000u));
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const uint32_t y = pack_f16x2(vals[2 * i], vals[2 * i + 1]);
+      const float2 yf = __half22float2(*reinterpret_cast<const __half2*>(&y));
+      const float2 bf = __half22float2(*reinterpret_cast<const __half2*>(&packed[i]));
+      vals[2 * i] = __fadd_rn(yf.x, bf.x);
+      vals[2 * i + 1] = __fadd_rn(yf.y, bf.y);
+    }
+  }
+}
+
 // Bias epilogue on 32 consecutive output columns of one row (`vals` already carry alpha). The
 // result is what adding a bias tensor to the stored output gives: for 2-byte outputs the
 // product is first rounded to the output type, then the sum is formed in FP32 and rounded again
@@ -157,23 +179,36 @@ __device__ __forceinline__ void add_bias_32(float (&vals)[32], const void* bias,
       packed[i] = lo | (hi << 16);
     }
   }
-  if (out_dtype == kOutBf16) {
+  add_packed_bias_32(vals, packed, out_dtype);
+}
+
+// The whole bias row of a tile (up to 256 columns of a 2-byte type) over the lanes of a warp: lane l
+// holds columns col0 + 8 * l onwards. Loaded before the wait for the accumulator, so that its latency
+// hides behind the main loop; asked for chunk by chunk in the epilogue it was exposed eight times
+// per tile, 3 us, while tensor memory waited to be released.
+__device__ __forceinline__ uint4 load_bias_row(const void* bias, int col0, int n, int lane) {
+  const uint16_t* b = static_cast<const uint16_t*>(bias) + col0 + lane * 8;
+  const int left = n - (col0 + lane * 8);
+  if (left >= 8 && (reinterpret_cast<uintptr_t>(b) & 15) == 0)
+    return __ldg(reinterpret_cast<const uint4*>(b));
+  uint32_t w[4];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const uint32_t y = pack_bf16x2(vals[2 * i], vals[2 * i + 1]);
-      vals[2 * i] = __fadd_rn(__uint_as_float(y << 16), __uint_as_float(packed[i] << 16));
-      vals[2 * i + 1] = __fadd_rn(__uint_as_float(y & 0xFFFF0000u), __uint_as_float(packed[i] & 0xFFFF0000u));
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const uint32_t y = pack_f16x2(vals[2 * i], vals[2 * i + 1]);
-      const float2 yf = __half22float2(*reinterpret_cast<const __half2*>(&y));
-      const float2 bf = __half22float2(*reinterpret_cast<const __half2*>(&packed[i]));
-      vals[2 * i] = __fadd_rn(yf.x, bf.x);
-      vals[2 * i + 1] = __fadd_rn(yf.y, bf.y);
-    }
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t lo = (2 * i < left) ? __ldg(b + 2 * i) : 0u;
+    const uint32_t hi = (2 * i + 1 < left) ? __ldg(b + 2 * i + 1) : 0u;
+    w[i] = lo | (hi << 16);
   }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// add_bias_32 from such a row: the 32 columns from lane `first_lane` on (whole warps).
+__device__ __forceinline__ void add_bias_row_32(float (&vals)[32], const uint4& row, int first_lane,
+                                                int out_dtype) {
+  const uint32_t w[4] = {row.x, row.y, row.z, row.w};
+  uint32_t packed[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) packed[i] = __shfl_sync(0xffffffffu, w[i & 3], first_lane + (i >> 2));
+  add_packed_bias_32(vals, packed, out_dtype);
 }
 
 // Same for a single output value (column `col`).
@@ -451,6 +486,10 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap map_a,
       tile_coords(local, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
       const int acc = iter % T::kAccStages;
       const uint32_t acc_phase = (iter / T::kAccStages) & 1;
+      uint4 bias_row = make_uint4(0, 0, 0, 0);
+      if constexpr (BIAS) {
+        if (p.use_tma_store) bias_row = load_bias_row(p.bias, tn * BN, p.n, lane);
+      }
       // The epilogue warps meet at barriers in the TMA-store path, so they agree on the
       // outcome of the wait before going on.
       if (!epilogue_bar_and(mbar_wait_bounded(&acc_full_bar[acc], acc_phase, abort_flag))) {
@@ -489,7 +528,7 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap map_a,
 #pragma unroll
               for (int i = 0; i < 32; ++i) vals[i] = __uint_as_float(cur[i]) * alpha;
               if constexpr (BIAS)
-                add_bias_32(vals, p.bias, p.out_dtype, tn * BN + pass * 128 + cc * 32, p.n);
+                add_bias_row_32(vals, bias_row, pass * 16 + cc * 4, p.out_dtype);
               uint32_t packed[16];
               if (p.out_dtype == kOutBf16) {
 #pragma unroll

@@ -421,6 +421,10 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       if constexpr (SCATTER) tm = scatter_tile_row(tm, p.tiles_m, sc.world);
       const int acc = iter % T::kAccStages;
       const uint32_t acc_phase = (iter / T::kAccStages) & 1;
+      uint4 bias_row = make_uint4(0, 0, 0, 0);
+      if constexpr (BIAS) {
+        if (p.use_tma_store) bias_row = load_bias_row(p.bias, tn * BN, p.n, lane);
+      }
       if (!epilogue_bar_and(mbar_wait_bounded_cluster(&acc_full_bar[acc], acc_phase, abort_flag))) {
         *abort_flag = 1;
         if (p.status && lane == 0) atomicMax(p.status, kStatusEpilogueTimeout);
@@ -591,7 +595,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
             float vals[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) vals[i] = __uint_as_float(raw[cc][i]) * alpha;
-            add_bias_32(vals, p.bias, p.out_dtype, tn * BN + half * 128 + cc * 32, p.n);
+            add_bias_row_32(vals, bias_row, half * 16 + cc * 4, p.out_dtype);
 #pragma unroll
             for (int i = 0; i < 16; ++i)
               packed[cc * 16 + i] = (p.out_dtype == kOutBf16)
