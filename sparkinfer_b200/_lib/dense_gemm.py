@@ -206,8 +206,8 @@ def _dense_gemm_launch_functional_fake(
 
 
 def _select_default_mma_tiler_mn(m: int, n: int, sm_count: int) -> Tuple[int, int]:
-    """Tile the kernel would pick for (m, n) on ``sm_count`` SMs: 128 rows by the width with
-    the fewest waves x per-tile cost (same model as the C side)."""
+    """Single-CTA tile for (m, n) on ``sm_count`` SMs when nothing is known of K: 128 rows by the
+    width with the fewest waves x per-tile cost (the library's own choice weighs K as well)."""
     best, best_cost = 128, None
     tiles_m = -(-m // 128)
     for bn in (256, 192, 128, 64):

@@ -15,26 +15,6 @@ thread_local char g_last_error[256] = "";
 
 namespace {
 
-// Tile width: fewest (waves x per-tile cost). The per-tile cost model is the bytes one k-step
-// pulls through shared memory, (128 + BN) rows of 128 bytes, which tracks both the MMA time
-// (proportional to BN) and the operand traffic.
-int choose_block_n(int64_t m, int64_t n, int sms) {
-  static const int candidates[] = {256, 192, 128, 64};
-  const int64_t tiles_m = (m + 127) / 128;
-  int best = 128;
-  double best_cost = 1e300;
-  for (int bn : candidates) {
-    const int64_t tiles = tiles_m * ((n + bn - 1) / bn);
-    const int64_t waves = (tiles + sms - 1) / sms;
-    const double cost = double(waves) * (128 + bn);
-    if (cost < best_cost) {
-      best_cost = cost;
-      best = bn;
-    }
-  }
-  return best;
-}
-
 template <int KIND, int BN, bool BIAS>
 int launch_gemm_impl(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_c,
                      const GemmParams& p, int grid, cudaStream_t stream) {
@@ -182,6 +162,53 @@ PairTailPlan plan_pair_tail(int kind, int64_t m, int64_t n, int64_t k, int64_t g
   return t;
 }
 
+// The tile of an unforced problem: 64, 128, 192 or 256 columns on the single-CTA kernel, or
+// B12X_B200_BLOCK_N_PAIR. Least estimated time, rounds x (k-tiles x step + round) + fixed, in units
+// of 10 ns. A step is one 128-byte k-tile of a tile, a round what a tile costs besides (filling the
+// pipeline, the part of the epilogue the next tile waits for); a pair tile split along K adds `tail`.
+// The numbers are a fit to 44 shapes x 5 tiles per kind (M 65..6000, N 512..40000, K 512..18432,
+// device time, weights from HBM); the choice is within 0.6 % of the best tile on average (15 % at
+// worst), where fewest rounds x (128 + width) with two thirds of a round of pair tiles going to the
+// pair kernel was 8 % (MXFP8, FP8) and 12 % (NVFP4) off. Examples, before -> now in us: MXFP8
+// 84 x 35840 x 512 13.4 -> 8.9, 3353 x 1280 x 1024 10.9 -> 8.7, NVFP4 300 x 18432 x 1024 13.1 -> 9.2,
+// 81 x 37760 x 3584 21.0 -> 18.1.
+int choose_tile(int kind, int64_t m, int64_t n, int64_t k, int64_t groups, int sms) {
+  struct Cost { int block_n; int step[3], round[3], fixed; };   // MXFP8, FP4, unscaled FP8
+  static const Cost costs[] = {
+      {64, {27, 29, 26}, {50, 43, 30}, 370},
+      {128, {30, 32, 29}, {54, 55, 47}, 370},
+      {192, {36, 37, 34}, {106, 114, 88}, 370},
+      {256, {45, 48, 36}, {198, 184, 146}, 370},
+      {B12X_B200_BLOCK_N_PAIR, {33, 33, 32}, {209, 215, 179}, 490},
+  };
+  constexpr int kTail = 700;
+  const bool fp4 = kind == B12X_B200_KIND_NVFP4 || kind == B12X_B200_KIND_MXFP4;
+  const int row = kind == B12X_B200_KIND_FP8 ? 2 : fp4 ? 1 : 0;
+  const int64_t k_tiles = (k + (fp4 ? 255 : 127)) / (fp4 ? 256 : 128);
+  int best = 128;
+  int64_t best_cost = INT64_MAX;
+  for (const Cost& c : costs) {
+    int64_t cost;
+    if (c.block_n == B12X_B200_BLOCK_N_PAIR) {
+      if (sms < 2) continue;
+      const int64_t tiles = ((m + 255) / 256) * ((n + 255) / 256) * groups;
+      const int64_t pairs = tiles < sms / 2 ? tiles : sms / 2;
+      const PairTailPlan tail = plan_pair_tail(kind, m, n, k, groups, sms);
+      const int64_t whole = tail.segments >= 2 ? tiles / pairs : (tiles + pairs - 1) / pairs;
+      cost = whole * (k_tiles * c.step[row] + c.round[row]) + c.fixed;
+      if (tail.segments >= 2) cost += k_tiles * c.step[row] / tail.segments + c.round[row] + kTail;
+    } else {
+      const int64_t tiles = ((m + 127) / 128) * ((n + c.block_n - 1) / c.block_n) * groups;
+      cost = (tiles + sms - 1) / sms * (k_tiles * c.step[row] + c.round[row]) + c.fixed;
+    }
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = c.block_n;
+    }
+  }
+  return best;
+}
+
 }  // namespace
 }  // namespace b12x_b200
 
@@ -252,14 +279,9 @@ int gemm_blockscaled_impl(int kind, const void* a, const void* sfa, const void* 
   const int sms = (sm_count > 0 && sm_count < info.sm_count) ? sm_count : info.sm_count;
   if (block_n == B12X_B200_BLOCK_N_PAIR && sms < 2)
     return fail(B12X_B200_ERR_UNSUPPORTED, "the CTA-pair kernel needs two SMs");
-  const int bn = block_n > 0 ? block_n : choose_block_n(m, n, sms);
-
-  // Problems with enough 256 x 256 pair tiles go to the CTA-pair kernel unless a tile width was
-  // forced. "Enough" is two thirds of the pairs: measured on 148 SMs the pair kernel wins from
-  // 56 tiles up (512 x 7168, 1024 x 4096, 256 x 18432) and loses at 28-32 tiles.
+  const int bn = block_n != 0 ? block_n : choose_tile(kind, m, n, k, groups, sms);
+  const bool use_pair = bn == B12X_B200_BLOCK_N_PAIR;
   const int64_t pair_tiles = ((m + 255) / 256) * ((n + 255) / 256) * groups;
-  const bool use_pair = (block_n == B12X_B200_BLOCK_N_PAIR) ||
-                        ((block_n == 0) && (sms >= 2) && (pair_tiles * 3 >= sms));
 
   CUtensorMap map_a, map_b;
   rc = make_operand_map(&map_a, a, uint64_t(m), uint64_t(row_bytes), 128, uint64_t(groups));
@@ -280,7 +302,7 @@ int gemm_blockscaled_impl(int kind, const void* a, const void* sfa, const void* 
   p.ldc = int(ldc);
   p.out_dtype = c_dtype;
   p.tiles_m = int((m + 127) / 128);
-  p.tiles_n = int((n + bn - 1) / bn);
+  p.tiles_n = use_pair ? int((n + 255) / 256) : int((n + bn - 1) / bn);
   p.k_atoms_total = scaled ? int((k + sf_vec * 4 - 1) / (sf_vec * 4)) : 0;
   p.group_m = 16;
   p.bias = epilogue ? epilogue->bias : nullptr;
@@ -403,10 +425,9 @@ int64_t tiled_workspace_bytes(int kind, int64_t m, int64_t n, int64_t k, int64_t
   DeviceInfo info;
   if (device_info(&info) != B12X_B200_OK) return -1;
   const int sms = (sm_count > 0 && sm_count < info.sm_count) ? sm_count : info.sm_count;
-  const int64_t pair_tiles = ((m + 255) / 256) * ((n + 255) / 256) * groups;
-  const bool use_pair = (block_n == B12X_B200_BLOCK_N_PAIR) ||
-                        ((block_n == 0) && (sms >= 2) && (pair_tiles * 3 >= sms));
-  if (!use_pair || sms < 2) return 0;
+  // For an unforced problem what the CTA-pair kernel would use, whether or not choose_tile takes
+  // it: a workspace sized once stays large enough when the choice is tuned.
+  if ((block_n != 0 && block_n != B12X_B200_BLOCK_N_PAIR) || sms < 2) return 0;
   const PairTailPlan tp = plan_pair_tail(kind, m, n, k, groups, sms);
   return tp.segments >= 2 ? int64_t(tp.bytes) : 0;
 }

@@ -1,0 +1,44 @@
+"""The tile an unforced GEMM gets (single-CTA widths 64 to 256, CTA pair with and without split
+leftover tiles): FP32 outputs of the unforced call and of every forced tile against the 128-column
+tile. All sum the same products in FP32, so they differ by at most 2 * K * 2^-24 of the sum of
+magnitudes, which for these operands is below sqrt(K) times the largest result."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from sparkinfer_b200 import _native
+from test_decode_split_gpu import DEV, _operand
+
+pytestmark = pytest.mark.gpu
+
+
+# Few rows against a wide weight, short and long K, one and several rounds, ragged edges, and
+# shapes whose leftover pair tiles are split along K (80, 78 and 75 pair tiles on 74 pairs).
+@pytest.mark.parametrize("m,n,k", [
+    (65, 640, 512), (81, 37768, 512), (128, 4096, 4096), (129, 2000, 800), (300, 18432, 1024),
+    (1100, 920, 7168), (3353, 1280, 1024), (2048, 2560, 2048), (1536, 3328, 1024), (256, 19200, 1024)])
+@pytest.mark.parametrize("kind", [_native.KIND_MXFP8, _native.KIND_NVFP4, _native.KIND_FP8])
+@pytest.mark.parametrize("groups", [1, 2])
+def test_tiles_agree(kind, m, n, k, groups):
+    from sparkinfer_b200._lib import launch
+
+    if groups == 2 and m > 1000:
+        pytest.skip("one size of group is enough for the large shapes")
+    gen = torch.Generator(device=DEV).manual_seed(m + n + k)
+    parts = [(_operand(kind, m, k, gen), _operand(kind, n, k, gen)) for _ in range(groups)]
+    a, sfa, b, sfb = (torch.cat([p[i][j].reshape(-1) for p in parts]) for i in (0, 1) for j in (0, 1))
+    scales = (None, None) if kind == _native.KIND_FP8 else (sfa, sfb)
+    outs = {}
+    for block_n in (128, 0, 64, 192, 256, _native.BLOCK_N_PAIR):
+        c = torch.full((groups, m, n), float("nan"), dtype=torch.float32, device=DEV)
+        launch.gemm_blockscaled(kind, a, scales[0], b, scales[1], c, None, m, n, k, groups=groups,
+                                block_n=block_n, small_m=False)
+        outs[block_n] = c
+    launch.check_kernel_status(DEV)
+    ref = outs[128]
+    bound = 2.0 * k * 2.0 ** -24 * k ** 0.5 * float(ref.abs().max())
+    for block_n, c in outs.items():
+        assert not torch.isnan(c).any(), block_n
+        assert float((c - ref).abs().max()) <= bound, block_n
