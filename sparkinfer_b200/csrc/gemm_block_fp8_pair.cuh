@@ -84,7 +84,7 @@ gemm_block_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   if (threadIdx.x == 0) {
     for (int s = 0; s < T::kStages; ++s) {
       mbar_init(&full_bar[s], leader ? 2 : 1);  // own copies (+ the peer's, relayed)
-      mbar_init(&empty_bar[s], 2);              // one commit per half
+      mbar_init(&empty_bar[s], leader ? 2 : 1); // one commit per half (peer: the leader's producer)
     }
     for (int b = 0; b < T::kBuffers; ++b) {
       mbar_init(&part_full_bar[b], 1);
@@ -124,6 +124,7 @@ gemm_block_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a,
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    bool wrapped = false;   // the stages have been used before
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
       int tm, tn;
       tile_coords(tile, p.tiles_m, p.tiles_n, p.group_m, tm, tn);
@@ -137,6 +138,8 @@ gemm_block_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           break;
         }
         if (elect_one()) {
+          // The issuers free a stage in the leader, which passes it on to the peer.
+          if (leader && wrapped) mbar_arrive_cluster(map_to_cta(smem_addr_u32(&empty_bar[stage]), 1));
           uint8_t* st = smem + stage * T::kStageBytes;
           mbar_arrive_expect_tx(&full_bar[stage], T::kStageBytes);
           tma_load_2d(st, &map_a, &full_bar[stage], kb * 128, m0);
@@ -145,7 +148,7 @@ gemm_block_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a,
                       n0 + T::kHalf);
         }
         __syncwarp();
-        if (++stage == T::kStages) { stage = 0; phase ^= 1; }
+        if (++stage == T::kStages) { stage = 0; phase ^= 1; wrapped = true; }
       }
     }
   } else if (warp == 1 && !leader) {
@@ -193,7 +196,7 @@ gemm_block_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           for (int j = 0; j < 4; ++j)
             tc_mma_f8_pair(buf * T::kHalf, adesc + 2 * j, bdesc + 2 * j, idesc, j > 0 ? 1u : 0u);
           tc_commit_pair_both(smem_addr_u32(&part_full_bar[buf]));
-          tc_commit_pair_both(smem_addr_u32(&empty_bar[stage]));
+          tc_commit_pair(smem_addr_u32(&empty_bar[stage]));
         }
         __syncwarp();
         if (++stage == T::kStages) { stage = 0; phase ^= 1; }

@@ -12,7 +12,9 @@
 //   producer (each CTA)  : wait own empty[s] -> arm own full[s], issue own loads
 //   relay (peer, warp 1) : wait own full[s]  -> arrive on the leader's full[s]
 //   issuer (leader, w 1) : wait own full[s] -> scale copies + 4 MMAs for the pair -> one
-//                          tcgen05.commit to empty[s] of both CTAs
+//                          tcgen05.commit to own empty[s]; the leader's producer, which waits for
+//                          it anyway, arrives on the peer's empty[s] (a second commit per stage
+//                          costs the issuing thread, which paces the kernel, 3-5 %)
 //   epilogue (each CTA)  : wait own acc_full (committed by the leader to both CTAs) -> pull own
 //                          128 x 256 accumulator into registers -> arrive on the leader's
 //                          acc_empty -> convert, stage in swizzled shared memory, TMA store
@@ -239,6 +241,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
+    bool wrapped = false;   // the stages have been used before
     PairWork w;
     for (int it = 0; ok && pair_work(it, pair, num_pairs, num_tiles, k_tiles, tail.segments, w); ++it) {
       int tm, tn, grp, local;
@@ -255,6 +258,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           break;
         }
         if (elect_one()) {
+          if (leader && wrapped) mbar_arrive_cluster(map_to_cta(smem_addr_u32(&empty_bar[stage]), 1));
           uint8_t* st = smem + stage * T::kStageBytes;
           uint64_t* bar = &full_bar[stage];
           mbar_arrive_expect_tx(bar, T::kABytes + T::kBBytes);
@@ -263,7 +267,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
                       n0 + static_cast<int>(rank) * (BN / 2), grp);
         }
         __syncwarp();
-        if (++stage == T::kStages) { stage = 0; phase ^= 1; }
+        if (++stage == T::kStages) { stage = 0; phase ^= 1; wrapped = true; }
       }
     }
   } else if (warp == 6 && !T::kScaled) {
@@ -400,8 +404,9 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
               tc_mma_nvf4_pair(d_taddr, adesc + 2 * j, bdesc + 2 * j, idesc_base, accumulate,
                                T::kSfaCol0 + j * 4, T::kSfbCol0 + j * T::kSfbRowAtoms * 4);
           }
-          // Free the stage in both CTAs; publish the accumulator to both after the last step.
-          tc_commit_pair_both(smem_addr_u32(&empty_bar[stage]));
+          // Free the stage (the leader's producer passes it on to the peer); publish the
+          // accumulator to both CTAs after the last step.
+          tc_commit_pair(smem_addr_u32(&empty_bar[stage]));
           if (kt == w.kt_end - 1) tc_commit_pair_both(smem_addr_u32(&acc_full_bar[acc]));
         }
         __syncwarp();

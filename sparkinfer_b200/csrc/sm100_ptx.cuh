@@ -435,13 +435,10 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t cluster_addr) {
                : "memory");
 }
 
-// The same with one arrival in each CTA of the pair, on the mbarrier at `smem_addr`'s offset.
+// One arrival in each CTA of the pair, on the mbarrier at `smem_addr`'s offset.
 __device__ __forceinline__ void tc_commit_pair_both(uint32_t smem_addr) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 "
-      "[%0], %1;"
-      ::"r"(smem_addr), "h"(static_cast<uint16_t>(3))
-      : "memory");
+  tc_commit_pair(smem_addr);
+  tc_commit_pair(map_to_cta(smem_addr, 1));
 }
 
 // Scale atom copy executed in both CTAs of the pair: each reads its own shared memory at the
