@@ -95,10 +95,11 @@ def _call_on(index: int, fn, *args) -> int:
 
 def plain_eager(*tensors: torch.Tensor | None) -> bool:
     """Whether a call on these tensors can go straight to the launcher: ordinary CUDA tensors with
-    nothing that listens to operators (tracing, dispatch modes, functorch transforms, forward-mode
+    nothing that listens to operators (tracing, function or dispatch modes, functorch, forward-mode
     differentiation, a graph being recorded for one of them). Otherwise it belongs to the
     registered custom op, which all of these know how to treat."""
     if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() != 0
+            or torch._C._len_torch_function_stack() != 0
             or torch._C._get_tracing_state() is not None
             or torch._C._functorch.peek_interpreter_stack() is not None
             or torch.autograd.forward_ad._current_level >= 0):

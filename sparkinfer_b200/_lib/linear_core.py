@@ -55,8 +55,9 @@ def pad_columns(rows: torch.Tensor, width: int) -> torch.Tensor:
 def multipliable_rows(rows: torch.Tensor, width: int) -> torch.Tensor:
     """``rows [T, K]`` for a weight padded to ``width`` columns. The kernels read K columns and
     take the weight's longer rows as a pitch, so nothing is padded here, unless the rows do not
-    start where their 16-byte loads can: the padded copy does."""
-    if rows.shape[1] != width and rows.data_ptr() % 16 != 0:
+    start where their 16-byte loads can or end inside a scale block: the padded copy does not."""
+    k = rows.shape[1]
+    if k != width and (k > width or k % SCALE_BLOCK or rows.data_ptr() % 16):
         return pad_columns(rows, width)
     return rows.contiguous()
 

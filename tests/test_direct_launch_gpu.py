@@ -67,3 +67,17 @@ def test_a_source_that_needs_gradients_keeps_the_op_route():
     assert tracked.requires_grad and torch.equal(tracked.detach(), plain)
     with torch.no_grad():
         assert not run(x.clone().requires_grad_(), None).requires_grad
+
+
+# Ragged K without a padded copy: rows that start on and off a 16-byte boundary, K beside and inside
+# a 128-element step, on the decode and the tiled kernels.
+@pytest.mark.parametrize("which", ["mxfp8", "tensor_fp8"])
+@pytest.mark.parametrize("m,k", [(3, 32), (40, 96), (40, 2080), (100, 160), (300, 1056)])
+def test_ragged_k_on_any_alignment(which, m, k):
+    run, source_dtype = _linear(which, k)
+    gen = torch.Generator(device=DEV).manual_seed(m + k)
+    x = torch.randn((m, k), device=DEV, generator=gen).to(source_dtype)
+    shifted = torch.empty(m * k + 1, dtype=source_dtype, device=DEV)[1:].view(m, k)
+    shifted.copy_(x)
+    assert shifted.data_ptr() % 16 != 0
+    assert torch.equal(run(x, None), run(shifted, None))
