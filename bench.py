@@ -62,7 +62,7 @@ NCU_TRAFFIC_BYTES = {
     "cfg0_nvfp4_128x4096x4096": 9_762_816 + 0,
     "cfg1_nvfp4_decode_m16": 33_151_232 + 256,
     "cfg2_mxfp8_prefill": 286_378_496 + 115_882_496,
-    "cfg3_block_fp8_colpar": 298_083_840 + 131_562_752,
+    "cfg3_block_fp8_colpar": 197_302_272 + 134_139_392,
     "cfg4_nvfp4_rowpar": 223_142_656 + 62_427_648,
 }
 
