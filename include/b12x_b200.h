@@ -214,13 +214,16 @@ int b12x_b200_gemm_linear(int kind, int decode, const void* x, const void* sf_x,
  *
  * Ordering on one stream. The kernel is launched with programmatic stream serialization: it
  * may start while the kernel launched just before it on the same stream is still running, if
- * that kernel releases its dependents early. In this library the decode GEMMs do, and the row
- * quantizers do for matrices of at most 128 rows. The decode GEMM reads x, sf_x and alpha and
+ * that kernel releases its dependents early. In this library the block-scaled decode GEMMs do at
+ * once, the row quantizers do at once for matrices of at most 128 rows, and the block-FP8 GEMM of
+ * few rows does when its own predecessor has completed. The decode GEMM reads x, sf_x and alpha and
  * writes c and the workspace only after its predecessor has completed. A weight of more than
- * 128 rows is streamed at once (no kernel of this library that releases early can have written
- * it); a weight of 128 rows or fewer is streamed after the predecessor has completed, like the
- * other operands. A foreign kernel that releases its dependents early (griddepcontrol /
- * cudaTriggerProgrammaticLaunchCompletion) must not be the writer of w or sf_w.
+ * 128 rows is streamed at once; a weight of 128 rows or fewer is streamed after the predecessor has
+ * completed, like the other operands. So a kernel that releases its dependents early must not have
+ * written w or sf_w of more than 128 rows: a foreign one (griddepcontrol /
+ * cudaTriggerProgrammaticLaunchCompletion), or a row quantizer of this library called on slabs of
+ * at most 128 rows of the weight. If one has, launch something that does not release early between
+ * it and the decode GEMM, or wait for the stream.
  */
 int64_t b12x_b200_gemm_smallm_workspace_bytes(int kind, int64_t m, int64_t n, int64_t k,
                                               int sm_count);
@@ -354,6 +357,9 @@ int b12x_b200_gemm_blockscaled_smallm_noalloc(int kind, const void* x, const voi
  *   a   [M, K] E4M3, K-major      sfa [M, K/128] FP32, contiguous
  *   b   [N, K] E4M3, K-major      sfb [N/128, K/128] FP32, contiguous
  *   N and K must be multiples of 128. Other arguments as for b12x_b200_gemm_blockscaled.
+ *
+ * Ordering on one stream: that of an ordinary launch for every M. All operands may be the output of
+ * the kernel launched just before, whether or not it releases its dependents early.
  */
 int b12x_b200_gemm_block_fp8(const void* a, const float* sfa, const void* b, const float* sfb,
                              void* c, int c_dtype, const float* alpha, int64_t m, int64_t n,

@@ -140,7 +140,6 @@ int run_block_fp8_small(const BlockFp8SmallPlan& pl, const void* a, const float*
   p.k_blocks = pl.k_blocks;
   p.split = pl.split;
   p.packed_store = (c_dtype != B12X_B200_FP32 && aligned16(c) && ldc % 8 == 0) ? 1 : 0;
-  p.wait_for_weights = n <= kEarlyReleaseRows ? 1 : 0;
   switch (pl.m_pad) {
     case 16: return launch_block_fp8_small<16>(a, b, p, k, pl.grid, stream);
     case 32: return launch_block_fp8_small<32>(a, b, p, k, pl.grid, stream);

@@ -32,9 +32,14 @@
 // Threads: warp 0 weight producer (and barrier set-up), warp 1 MMA issuer and TMEM owner, warp 2
 // activation producer, warp 3 scales, then four promotion warps per 16 or 32 activation rows, which
 // keep the sums in registers (with all of 64 rows in one group of four warps, each waits too long
-// for its own tensor-memory loads: 64 x 47232 x 2560 33 us instead of 27). Launched with
-// programmatic stream serialization; what may be a predecessor's output is only touched after
-// griddepcontrol.wait (the same contract as the block-scaled decode kernel).
+// for its own tensor-memory loads: 64 x 47232 x 2560 33 us instead of 27).
+//
+// Order on the stream: that of an ordinary launch. The kernel is launched with programmatic stream
+// serialization, but every operand, the weight too, is read behind griddepcontrol.wait: an FP32-scaled
+// weight is often written by kernels that are not this library's, and one that releases its
+// dependents early would otherwise still be writing it. (The block-scaled decode kernel streams its
+// weight earlier, on a condition its callers know.) The next grid is released behind the wait as
+// well, so that it cannot start beside a grid that this one itself has to wait for.
 #pragma once
 
 #include "gemm_blockscaled.cuh"
@@ -75,7 +80,6 @@ struct BlockFp8SmallParams {
   int tiles, k_blocks;
   int split;             // CTAs of a cluster = CTAs per tile
   int packed_store;      // 2-byte outputs with 16-byte aligned rows
-  int wait_for_weights;  // the weight may be a predecessor's fresh output (few rows)
 };
 
 // Eight output rows x 32 columns of a warp (lane = column): scale, bias, round, store.
@@ -136,8 +140,6 @@ gemm_block_fp8_smallm_kernel(const __grid_constant__ CUtensorMap map_w,
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  grid_launch_dependents();
-
   // This CTA: k-blocks [kb_begin, kb_end) of tiles tile0, tile0 + tile_step, ... (one tile when
   // it is split).
   const int rank = static_cast<int>(blockIdx.x) % p.split;
@@ -168,7 +170,8 @@ gemm_block_fp8_smallm_kernel(const __grid_constant__ CUtensorMap map_w,
     }
     __syncwarp();
     asm volatile("barrier.cta.arrive 3, %0;" ::"n"(T::kThreads) : "memory");
-    if (p.wait_for_weights) grid_dependency_wait();
+    grid_dependency_wait();    // the weight may come from the previous grid
+    grid_launch_dependents();  // every CTA of which has finished by now
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;

@@ -30,9 +30,10 @@
 // griddepcontrol.launch_dependents at once, so the next grid's CTAs are placed as soon as this
 // grid's CTAs leave their SMs and run their prologue and first weight loads while this grid is
 // still finishing. The weight producer starts streaming immediately when the weight has more
-// than 128 rows: the only kernels that release their dependents early are this one (output of
-// at most 128 rows) and the row quantizers (only for matrices of at most 128 rows), so such a
-// weight cannot be a predecessor's output still being written. The warps that read activations
+// than 128 rows: the only kernels that release their dependents early are this one and the
+// block-FP8 one of few rows (outputs of at most 128 rows) and the row quantizers (only for matrices
+// of at most 128 rows), so such a weight is no predecessor's whole output still being written (a
+// caller who lets slabs of it be written that way orders the calls). The warps that read activations
 // or alpha, or write C, partials or counters, wait for the predecessor to finish
 // (griddepcontrol.wait) first, and so does the weight producer for a weight of 128 rows or fewer.
 // Tensor memory is addressed relative to the allocation's base column and only as many columns
@@ -439,9 +440,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w,
     }
     __syncwarp();
     setup_bar_arrive(blockDim.x);
-    // A weight of more than 128 rows is never the output of a predecessor that releases its
-    // dependents early (decode GEMMs write at most 128 rows, the row quantizers release early
-    // only for matrices of at most 128 rows), so its stream starts at once.
+    // A weight of more than 128 rows is not the output of a predecessor that releases its
+    // dependents early (see the top of this file), so its stream starts at once.
     if (p.wait_for_weights) grid_dependency_wait();
     int stage = 0;
     uint32_t phase = 0;

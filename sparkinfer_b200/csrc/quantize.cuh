@@ -210,10 +210,12 @@ __device__ __forceinline__ void quantize_mxfp8_chunk(const QuantChunk& c, const 
 //     was still running; nothing is read or written before the predecessor has completed.
 //   - griddepcontrol.launch_dependents, only when the quantized matrix has at most 128 rows
 //     (early_release): the next kernel on the stream, if it too was launched with programmatic
-//     serialization, may start now. In this library that is the decode GEMM, which streams its
-//     weight operand at once and waits for this grid before it reads activations. A matrix of
-//     more than 128 rows may be somebody's weight operand, so its quantization never releases
-//     early (and the decode GEMM waits before streaming a weight of 128 rows or fewer).
+//     serialization, may start now. In this library that is the block-scaled decode GEMM, which
+//     streams its weight operand at once and waits for this grid before it reads activations (the
+//     block-FP8 GEMM of few rows waits before it reads anything). A matrix of more than 128 rows
+//     may be somebody's weight operand, so its quantization never releases early (and the decode
+//     GEMM waits before streaming a weight of 128 rows or fewer). A larger weight quantized in
+//     slabs of at most 128 rows is the caller's to order: see the C header.
 __device__ __forceinline__ void quant_grid_prologue(int early_release) {
   if (early_release) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
