@@ -87,10 +87,11 @@ __device__ __forceinline__ void store_block_fp8_rows8(const BlockFp8SmallParams&
                                                       int lane, float alpha, int row0, int col0,
                                                       float (&vals)[8]) {
   const int col = col0 + lane;
+  const float bias = p.bias != nullptr ? load_bias_1(p.bias, p.out_dtype, col, p.n) : 0.0f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     vals[i] *= alpha;
-    if (p.bias != nullptr) vals[i] = add_bias_1(vals[i], p.bias, p.out_dtype, col, p.n);
+    if (p.bias != nullptr) vals[i] = add_bias_1(vals[i], bias, p.out_dtype);
   }
   if (p.packed_store) {
     store_rows8_packed(p, reinterpret_cast<uint16_t*>(staging), lane, 0, row0, col0, vals);
@@ -272,12 +273,12 @@ gemm_block_fp8_smallm_kernel(const __grid_constant__ CUtensorMap map_w,
           const int row0 = (lane >> 3) * kRows;
           const int kb = base + (lane & 7);
           const bool live = kb < kb_end;
-          const float w = live ? __ldg(p.sfw + static_cast<size_t>(tile) * p.k_blocks + kb) : 0.0f;
+          const float w = live ? ld_global_f32(p.sfw + static_cast<size_t>(tile) * p.k_blocks + kb) : 0.0f;
           const float* src = p.sfx + static_cast<size_t>(row0) * p.k_blocks + kb;
           float x[kRows];
 #pragma unroll
           for (int i = 0; i < kRows; ++i)
-            x[i] = (live && row0 + i < p.m) ? __ldg(src + static_cast<size_t>(i) * p.k_blocks) : 0.0f;
+            x[i] = (live && row0 + i < p.m) ? ld_global_f32(src + static_cast<size_t>(i) * p.k_blocks) : 0.0f;
           if (!mbar_wait_bounded(&scale_empty_bar[slot], ((batch / T::kScaleSlots) & 1) ^ 1, abort_flag)) {
             *abort_flag = 1;
             if (p.status && lane == 0) atomicMax(p.status, kStatusProducerTimeout);

@@ -211,15 +211,22 @@ __device__ __forceinline__ void add_bias_row_32(float (&vals)[32], const uint4& 
   add_packed_bias_32(vals, packed, out_dtype);
 }
 
-// Same for a single output value (column `col`).
-__device__ __forceinline__ float add_bias_1(float v, const void* bias, int out_dtype, int col, int n) {
-  if (bias == nullptr || col >= n) return v;
-  if (out_dtype == kOutFp32) return __fadd_rn(v, __ldg(static_cast<const float*>(bias) + col));
-  const uint32_t b = __ldg(static_cast<const uint16_t*>(bias) + col);
-  if (out_dtype == kOutBf16)
-    return __fadd_rn(__bfloat162float(__float2bfloat16_rn(v)), __uint_as_float(b << 16));
+// The bias of one column as FP32, 0 from column n on. Coherent load: the kernels that start beside
+// their predecessor use it too.
+__device__ __forceinline__ float load_bias_1(const void* bias, int out_dtype, int col, int n) {
+  if (col >= n) return 0.0f;
+  if (out_dtype == kOutFp32) return ld_global_f32(static_cast<const float*>(bias) + col);
+  const uint32_t b = ld_global_u16(static_cast<const uint16_t*>(bias) + col);
+  if (out_dtype == kOutBf16) return __uint_as_float(b << 16);
   const __half_raw hr = {static_cast<unsigned short>(b)};
-  return __fadd_rn(__half2float(__float2half_rn(v)), __half2float(__half(hr)));
+  return __half2float(__half(hr));
+}
+
+// add_bias_32 for a single output value whose column has the bias `b`.
+__device__ __forceinline__ float add_bias_1(float v, float b, int out_dtype) {
+  if (out_dtype == kOutFp32) return __fadd_rn(v, b);
+  if (out_dtype == kOutBf16) return __fadd_rn(__bfloat162float(__float2bfloat16_rn(v)), b);
+  return __fadd_rn(__half2float(__float2half_rn(v)), b);
 }
 
 // Writes 32 consecutive output columns of one row of group `group`. `vals` already carry alpha.

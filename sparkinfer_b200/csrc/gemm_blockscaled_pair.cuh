@@ -546,7 +546,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap map_a,
               float o[4] = {sum[i].x * alpha, sum[i].y * alpha, sum[i].z * alpha, sum[i].w * alpha};
               if constexpr (BIAS) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) o[j] = add_bias_1(o[j], p.bias, p.out_dtype, col + j, p.n);
+                for (int j = 0; j < 4; ++j) 
+                  o[j] = add_bias_1(o[j], load_bias_1(p.bias, p.out_dtype, col + j, p.n), p.out_dtype);
               }
               const size_t idx = SCATTER ? static_cast<size_t>(row + row_shift) * p.ldc + col
                                          : static_cast<size_t>(grp) * p.c_group_elems +

@@ -323,7 +323,8 @@ struct FusedQuant {
 // inside, cost 0.9 us at M = 16 and 2.8 us at M = 64).
 template <bool EPI>
 __device__ __forceinline__ void emit_output(const SmallMParams& p, float alpha, int lane, int grp,
-                                            int mrow, int n_global, bool n_ok, float acc_value) {
+                                            int mrow, int n_global, bool n_ok, float acc_value,
+                                            float bias_value) {
   float v = acc_value * alpha;
   const size_t idx = static_cast<size_t>(grp) * p.c_group_elems +
                      static_cast<size_t>(mrow) * p.ldc + n_global;
@@ -338,7 +339,7 @@ __device__ __forceinline__ void emit_output(const SmallMParams& p, float alpha, 
     }
     return;
   } else {
-    if (p.bias != nullptr) v = add_bias_1(v, p.bias, p.out_dtype, n_global, p.n);
+    if (p.bias != nullptr) v = add_bias_1(v, bias_value, p.out_dtype);
     float stored = v;
     if (p.out_dtype == kOutBf16) {
       const __nv_bfloat16 h = __float2bfloat16_rn(v);
@@ -718,6 +719,10 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w,
         const int grp = tile / p.tiles_per_group;
         const int n_global = (tile - grp * p.tiles_per_group) * 128 + n_local;  // inside the group
         const bool n_ok = n_global < p.n;
+        float bias_value = 0.0f;   // of this lane's column; behind the wait above
+        if constexpr (EPI) {
+          if (p.bias != nullptr) bias_value = load_bias_1(p.bias, p.out_dtype, n_global, p.n);
+        }
         const size_t c_group0 = static_cast<size_t>(grp) * p.c_group_elems;
         int first_cta = 0, segments = 1, slot = 0;
         if (!whole) {
@@ -759,7 +764,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w,
               for (int r = 0; r < 8; ++r) {
                 vals[r] = __uint_as_float(raw[8 * h + r]) * alpha;
                 if constexpr (EPI) {  // bias only (a quantized output keeps the per-lane path)
-                  if (p.bias != nullptr) vals[r] = add_bias_1(vals[r], p.bias, p.out_dtype, n_global, p.n);
+                  if (p.bias != nullptr) vals[r] = add_bias_1(vals[r], bias_value, p.out_dtype);
                 }
               }
               store_rows8_packed(p, buf, lane, c_group0, c0 + 8 * h, col0, vals);
@@ -793,7 +798,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w,
               const int mrow = c0 + i;
               if constexpr (EPI) {
                 if (mrow < p.m)
-                  emit_output<true>(p, alpha, lane, grp, mrow, n_global, n_ok, __uint_as_float(raw[i]));
+                  emit_output<true>(p, alpha, lane, grp, mrow, n_global, n_ok, __uint_as_float(raw[i]),
+                                    bias_value);
               } else if (n_ok && mrow < p.m) {
                 const float v = __uint_as_float(raw[i]) * alpha;
                 const size_t idx = c_group0 + static_cast<size_t>(mrow) * p.ldc + n_global;
@@ -847,7 +853,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w,
                 for (int i = 0; i < 8; ++i) {
                   vals[i] = sum[i] * alpha;
                   if constexpr (EPI) {
-                    if (p.bias != nullptr) vals[i] = add_bias_1(vals[i], p.bias, p.out_dtype, n_global, p.n);
+                    if (p.bias != nullptr) vals[i] = add_bias_1(vals[i], bias_value, p.out_dtype);
                   }
                 }
                 store_rows8_packed(p, reinterpret_cast<uint16_t*>(staging) + quarter * 256, lane,
@@ -859,7 +865,8 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap map_w,
               for (int i = 0; i < 8; ++i) {
                 const int mrow = m0 + i;
                 if constexpr (EPI) {
-                  if (mrow < p.m) emit_output<true>(p, alpha, lane, grp, mrow, n_global, n_ok, sum[i]);
+                  if (mrow < p.m)
+                    emit_output<true>(p, alpha, lane, grp, mrow, n_global, n_ok, sum[i], bias_value);
                 } else if (n_ok && mrow < p.m) {
                   const float v = sum[i] * alpha;
                   const size_t idx = c_group0 + static_cast<size_t>(mrow) * p.ldc + n_global;

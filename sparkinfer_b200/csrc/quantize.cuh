@@ -54,9 +54,11 @@ __device__ __forceinline__ void unpack8<__half>(const uint4& raw, float (&out)[8
   }
 }
 
-__device__ __forceinline__ uint4 ld_nc_16(const void* p) {
+// Read once, so not kept in L1; coherent, since the source may have been written while this grid was
+// already running (it starts beside its predecessor).
+__device__ __forceinline__ uint4 ld_once_16(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;
@@ -169,7 +171,7 @@ __device__ __forceinline__ void quantize_mxfp8_chunk(const QuantChunk& c, const 
 #pragma unroll
   for (int j = 0; j < kQuantLoadsPerLane; ++j) {
     const bool live = kFull || (row_live && c.k_base + j * 256 < k);
-    raw[j] = live ? ld_nc_16(src_row + j * 256) : make_uint4(0, 0, 0, 0);
+    raw[j] = live ? ld_once_16(src_row + j * 256) : make_uint4(0, 0, 0, 0);
   }
   // Addresses for load 0; load j adds a constant (256 codes, 8 scale columns = 2 atoms).
   uint8_t* out_values = values + static_cast<int64_t>(c.row) * k + c.k_base;
@@ -276,7 +278,7 @@ __device__ __forceinline__ void quantize_nvfp4_chunk(const QuantChunk& c, const 
 #pragma unroll
   for (int j = 0; j < kQuantLoadsPerLane; ++j) {
     const bool live = kFull || (row_live && c.k_base + j * 256 < k);
-    raw[j] = live ? ld_nc_16(src_row + j * 256) : make_uint4(0, 0, 0, 0);
+    raw[j] = live ? ld_once_16(src_row + j * 256) : make_uint4(0, 0, 0, 0);
   }
   const float r = (gs == 0.0f) ? 0.0f : __frcp_rn(gs);
   // Block maxima: a block is the 16 elements of two neighbouring lanes.

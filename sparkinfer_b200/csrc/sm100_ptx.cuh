@@ -63,6 +63,21 @@ __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Loads of what a predecessor may have written while this grid was already running: coherent, and
+// never moved in front of the wait. (__ldg and ld.global.nc ask for data that stays as it is for
+// the whole life of the grid.)
+__device__ __forceinline__ float ld_global_f32(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ uint32_t ld_global_u16(const uint16_t* p) {
+  uint16_t v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+
 // ----------------------------------------------------------------------------------------
 // mbarrier
 // ----------------------------------------------------------------------------------------

@@ -53,3 +53,87 @@ def test_block_fp8_weight_written_just_before(m, n, k):
     launch.check_kernel_status(DEV)
     for i, out in enumerate(got):
         assert torch.equal(out, want[i % 2]), i
+
+
+# The activation scales (FP32, [M, 128] for K = 16384) are the output of the GEMM launched just before,
+# and so is the bias, the single row of a GEMM of one activation row. Both releases are early.
+@pytest.mark.parametrize("m", [1, 24, 64, 65])
+def test_block_fp8_scales_and_bias_written_just_before(m):
+    from sparkinfer_b200._lib import launch
+
+    n, k = 1152, 16384
+    gen = torch.Generator(device=DEV).manual_seed(m)
+    a, b = _codes(m, k, gen), _codes(n, k, gen)
+    sb = torch.rand((n // 128, k // 128), device=DEV, generator=gen) + 0.25
+    sa = torch.empty((m, k // 128), dtype=torch.float32, device=DEV)
+    bias = torch.empty((1, n), dtype=torch.bfloat16, device=DEV)
+    small = [_codes(rows, 512, gen) for rows in (m, k // 128, 1, n)]
+    ones = [torch.ones((rows, 4), device=DEV) for rows in (m, 1)]
+    weight_scales = [torch.rand((rows // 128, 4), device=DEV, generator=gen) for rows in (k // 128, n)]
+    alphas = [torch.tensor([v], device=DEV) for v in (1.0, -0.5)]
+
+    def write(alpha):
+        launch.gemm_block_fp8(small[2], ones[1], small[3], weight_scales[1], bias, alpha, 1, n, 512)
+        launch.gemm_block_fp8(small[0], ones[0], small[1], weight_scales[0], sa, alpha, m, k // 128, 512)
+
+    def multiply():
+        out = torch.empty((m, n), dtype=torch.bfloat16, device=DEV)
+        launch.gemm_block_fp8(a, sa, b, sb, out, None, m, n, k, bias=bias[0])
+        return out
+
+    want = []
+    for alpha in alphas:
+        write(alpha)
+        torch.cuda.synchronize()
+        want.append(multiply())
+        torch.cuda.synchronize()
+    assert not torch.equal(*want)
+    got = []
+    for i in range(ROUNDS):
+        torch.cuda._sleep(2_000_000)
+        write(alphas[i % 2])
+        got.append(multiply())
+    launch.check_kernel_status(DEV)
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 2]), i
+
+
+# The same for the bias of the block-scaled decode GEMM, on whole tiles and on tiles cut along K.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,k", [(1032, 512), (640, 8192)])
+def test_decode_bias_written_just_before(n, k, dtype):
+    from sparkinfer_b200 import _native
+    from sparkinfer_b200._lib import launch
+
+    gen = torch.Generator(device=DEV).manual_seed(n + k)
+    m = 7
+    tiles, atoms = -(-n // 128), k // 128
+    a, b, row = _codes(m, k, gen), _codes(n, k, gen), _codes(1, k, gen)
+    sfa = torch.full((atoms * 512,), 127, dtype=torch.uint8, device=DEV)
+    sfb = torch.full((tiles * atoms * 512,), 127, dtype=torch.uint8, device=DEV)
+    bias = torch.empty((1, n), dtype=dtype, device=DEV)
+    alphas = [torch.tensor([v], device=DEV) for v in (1.0, -0.5)]
+
+    def write(alpha):
+        launch.gemm_blockscaled(_native.KIND_MXFP8, row, sfa, b, sfb, bias, alpha, 1, n, k)
+
+    def multiply():
+        out = torch.empty((m, n), dtype=dtype, device=DEV)
+        launch.gemm_blockscaled(_native.KIND_MXFP8, a, sfa, b, sfb, out, None, m, n, k, bias=bias[0])
+        return out
+
+    want = []
+    for alpha in alphas:
+        write(alpha)
+        torch.cuda.synchronize()
+        want.append(multiply())
+        torch.cuda.synchronize()
+    assert not torch.equal(*want)
+    got = []
+    for i in range(ROUNDS):
+        torch.cuda._sleep(2_000_000)
+        write(alphas[i % 2])
+        got.append(multiply())
+    launch.check_kernel_status(DEV)
+    for i, out in enumerate(got):
+        assert torch.equal(out, want[i % 2]), i
