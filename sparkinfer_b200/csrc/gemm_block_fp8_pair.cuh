@@ -20,6 +20,14 @@
 // warp 3: with every promotion warp loading its own rows' scales each load touched 32 cache lines,
 // half of the load unit's time (one issuer and such loads: 561 us at 4096 x 18432 x 7168).
 //
+// Hand-shakes across the pair: a barrier that the other CTA (or the pair's tensor core) signals is
+// waited for with cluster-scope acquire, as in gemm_blockscaled_pair.cuh: the leader's full, empty and
+// part_empty, the peer's empty, part_full in both. Between the CTAs only asynchronous copies and
+// tensor memory change hands, never ordinary memory: a promotion warp's reads of a buffer have
+// completed (tcgen05.wait::ld) and are ordered before its arrival by tcgen05.fence::before_thread_sync,
+// the issuer's MMA after its wait by the fence::after_thread_sync. The arrivals therefore keep the
+// default scope: with cluster-scope release on part_empty 4096 x 18432 x 7168 takes 950 us, not 487.
+//
 // Measured (device time, single-CTA kernel -> this one): 4096 x 18432 x 7168 535 -> 499 us (2.17
 // PFLOP/s), 8192 x 4096 x 4096 162 -> 145, 512 x 4096 x 7168 39.1 -> 37.1. What is left: without the
 // promotion FMAs it runs in 414 us, without tensor-memory loads too in 388, MMAs and operand loads
@@ -131,7 +139,7 @@ gemm_block_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       const int m0 = tm * 256 + static_cast<int>(rank) * T::BM;
       const int n0 = tn * T::BN + static_cast<int>(rank) * (T::kHalf / 2);
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (!mbar_wait_bounded(&empty_bar[stage], phase ^ 1, abort_flag)) {
+        if (!mbar_wait_bounded_cluster(&empty_bar[stage], phase ^ 1, abort_flag)) {
           *abort_flag = 1;
           if (p.status && lane == 0) atomicMax(p.status, kStatusProducerTimeout);
           ok = false;
@@ -183,8 +191,8 @@ gemm_block_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         const uint64_t adesc = make_kmajor_sw128_desc(st);
         const uint64_t bdesc = make_kmajor_sw128_desc(st + T::kABytes + half * T::kBHalfBytes);
         const uint32_t buf = (it & 1) * 2 + half;
-        if (!mbar_wait_bounded(&full_bar[stage], phase, abort_flag) ||
-            !mbar_wait_bounded(&part_empty_bar[buf], ((it >> 1) & 1) ^ 1, abort_flag)) {
+        if (!mbar_wait_bounded_cluster(&full_bar[stage], phase, abort_flag) ||
+            !mbar_wait_bounded_cluster(&part_empty_bar[buf], ((it >> 1) & 1) ^ 1, abort_flag)) {
           *abort_flag = 1;
           if (p.status && lane == 0) atomicMax(p.status, kStatusMmaTimeout);
           ok = false;
@@ -276,7 +284,7 @@ gemm_block_fp8_pair_kernel(const __grid_constant__ CUtensorMap map_a,
         const float scale = scales[slot * T::kScaleFloats +
                                    (half * T::kBatch + (kb & (T::kBatch - 1))) * T::kScalePitch +
                                    quarter * 32 + lane];
-        if (!ok || !mbar_wait_bounded(&part_full_bar[buf], (it >> 1) & 1, abort_flag)) {
+        if (!ok || !mbar_wait_bounded_cluster(&part_full_bar[buf], (it >> 1) & 1, abort_flag)) {
           *abort_flag = 1;
           if (p.status && lane == 0) atomicMax(p.status, kStatusEpilogueTimeout);
           ok = false;
