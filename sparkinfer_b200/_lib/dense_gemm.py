@@ -19,7 +19,6 @@ physical ``[L, M, N]`` storage.
 
 from __future__ import annotations
 
-import functools
 import os
 import logging
 import time
@@ -42,18 +41,18 @@ _MXFP6_AB_DTYPES = ("float6_e3m2fn", "float6_e2m3fn")
 _C_DTYPES = {"bfloat16": torch.bfloat16, "float16": torch.float16, "float32": torch.float32}
 _KERNEL_BLOCK_N = (64, 128, 192, 256)
 _ALPHA_ONE_CACHE: dict[tuple[str, int | None], torch.Tensor] = {}
+_NUM_SM: dict[int, int] = {}
 
 
-def get_num_sm(device: torch.device) -> int:
-    index = getattr(device, "index", None)
-    if index is not None:
-        return _num_sm(index)
-    return torch.cuda.get_device_properties(device).multi_processor_count
-
-
-@functools.lru_cache(maxsize=64)
-def _num_sm(index: int) -> int:
-    return torch.cuda.get_device_properties(index).multi_processor_count
+def get_num_sm(device: torch.device | str | int) -> int:
+    # Kept per index for eager calls. Tracing reads the property itself (a guarded constant there).
+    if not isinstance(device, torch.device) or device.index is None or torch.compiler.is_compiling():
+        return torch.cuda.get_device_properties(device).multi_processor_count
+    count = _NUM_SM.get(device.index)
+    if count is None:
+        count = torch.cuda.get_device_properties(device).multi_processor_count
+        _NUM_SM[device.index] = count
+    return count
 
 
 def _cached_alpha_one(device: torch.device | str) -> torch.Tensor:

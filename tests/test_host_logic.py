@@ -308,3 +308,22 @@ def test_grouped_fused_quant_host_checks_fire_before_any_launch():
         blockscaled.mm_fused_quant_a_grouped(src, b, sfb, groups=groups, positions=positions,
                                              cos_sin_cache=torch.zeros((8, 32), dtype=torch.float16),
                                              **rope)
+
+
+# ---------------------------------------------------------------------------------------
+# Host path of a call
+# ---------------------------------------------------------------------------------------
+@pytest.mark.parametrize("device", [torch.device("cuda", 1), torch.device("cuda"), "cuda:1", "cuda", 1])
+def test_num_sm_takes_every_form_of_a_device(monkeypatch, device):
+    from types import SimpleNamespace
+
+    from sparkinfer_b200._lib import dense_gemm
+
+    def properties(d):
+        assert isinstance(d, (torch.device, str, int))
+        return SimpleNamespace(multi_processor_count=148)
+
+    monkeypatch.setattr(torch.cuda, "get_device_properties", properties)
+    monkeypatch.setattr(dense_gemm, "_NUM_SM", {})
+    for _ in range(2):
+        assert dense_gemm.get_num_sm(device) == 148
