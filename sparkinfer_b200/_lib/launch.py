@@ -16,10 +16,13 @@ import torch
 from .. import _native
 
 # torch's own accessors without their Python wrappers: at a few microseconds per kernel the host
-# time of a call is most of a decode step, and each wrapper costs as much as a whole check here.
-_current_device = torch._C._cuda_getDevice
-_current_raw_stream = torch._C._cuda_getCurrentRawStream
-_capturing = torch._C._cuda_isCurrentStreamCapturing
+# time of a call is most of a decode step, and each wrapper costs as much as a whole check here. A
+# torch built without CUDA has none of them (and no CUDA tensor that would get here).
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+_current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream",
+                              lambda index: torch.cuda.current_stream(index).cuda_stream)
+_capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing",
+                     torch.cuda.is_current_stream_capturing)
 
 _STATUS_LOCK = Lock()
 _STATUS: dict[int, torch.Tensor] = {}

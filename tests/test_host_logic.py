@@ -327,3 +327,18 @@ def test_num_sm_takes_every_form_of_a_device(monkeypatch, device):
     monkeypatch.setattr(dense_gemm, "_NUM_SM", {})
     for _ in range(2):
         assert dense_gemm.get_num_sm(device) == 148
+
+
+def test_the_package_imports_on_a_torch_without_cuda():
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    code = ("import torch\n"
+            "for name in [n for n in dir(torch._C) if n.startswith('_cuda')]:\n"
+            "    delattr(torch._C, name)\n"
+            "import sparkinfer_b200._lib.launch\n"
+            "from sparkinfer_b200 import gemm, quantization\n")
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
+                          cwd=Path(__file__).resolve().parents[1])
+    assert done.returncode == 0, done.stderr[-2000:]
