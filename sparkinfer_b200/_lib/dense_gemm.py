@@ -45,13 +45,13 @@ _NUM_SM: dict[int, int] = {}
 
 
 def get_num_sm(device: torch.device | str | int) -> int:
-    # Kept per index for eager calls. Tracing reads the property itself (a guarded constant there).
-    if not isinstance(device, torch.device) or device.index is None or torch.compiler.is_compiling():
-        return torch.cuda.get_device_properties(device).multi_processor_count
-    count = _NUM_SM.get(device.index)
+    # Kept per device index. (A dict and not lru_cache, which torch.compile warns about.)
+    index = device.index if isinstance(device, torch.device) else None
+    count = _NUM_SM.get(index)
     if count is None:
         count = torch.cuda.get_device_properties(device).multi_processor_count
-        _NUM_SM[device.index] = count
+        if index is not None:
+            _NUM_SM[index] = count
     return count
 
 
