@@ -96,16 +96,25 @@ def _call_on(index: int, fn, *args) -> int:
         return fn(*args)
 
 
+# B12X_B200_DIRECT_LAUNCH=0: every call of dense_gemm and of the linears goes through its custom op.
+DIRECT_LAUNCH = _os.getenv("B12X_B200_DIRECT_LAUNCH", "1") != "0"
+
+_dispatch_modes = torch._C._len_torch_dispatch_stack
+_function_modes = torch._C._len_torch_function_stack
+_jit_tracing = torch._C._is_tracing
+_functorch_level = torch._C._functorch.peek_interpreter_stack
+_forward_ad = torch.autograd.forward_ad
+_profiler = torch.autograd.profiler
+
+
 def plain_eager(*tensors: torch.Tensor | None) -> bool:
-    """Whether a call on these tensors can go straight to the launcher: ordinary CUDA tensors with
-    nothing that listens to operators (tracing, function or dispatch modes, functorch, forward-mode
-    differentiation, a graph being recorded for one of them). Otherwise it belongs to the
-    registered custom op, which all of these know how to treat."""
-    if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() != 0
-            or torch._C._len_torch_function_stack() != 0
-            or torch._C._get_tracing_state() is not None
-            or torch._C._functorch.peek_interpreter_stack() is not None
-            or torch.autograd.forward_ad._current_level >= 0):
+    """Whether a linear's call on these tensors can go straight to the launcher: ordinary CUDA tensors
+    with nothing that listens to operators (tracing, function or dispatch modes, functorch,
+    forward-mode differentiation, the profiler, a graph being recorded for one of them). Otherwise it
+    belongs to the registered custom op, which all of these know how to treat."""
+    if (not DIRECT_LAUNCH or torch.compiler.is_compiling() or _dispatch_modes() != 0
+            or _function_modes() != 0 or _jit_tracing() or _functorch_level() is not None
+            or _forward_ad._current_level >= 0 or _profiler._is_profiler_enabled):
         return False
     grad = torch.is_grad_enabled()
     for t in tensors:

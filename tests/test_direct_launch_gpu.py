@@ -81,3 +81,22 @@ def test_ragged_k_on_any_alignment(which, m, k):
     shifted.copy_(x)
     assert shifted.data_ptr() % 16 != 0
     assert torch.equal(run(x, None), run(shifted, None))
+
+
+def test_the_switch_and_the_profiler_see_the_op(monkeypatch):
+    from sparkinfer_b200._lib import launch
+    from sparkinfer_b200.gemm.mxfp8_linear import _kernel
+
+    run, _ = _linear("mxfp8", 288)
+    x = torch.randn((5, 288), device=DEV, dtype=torch.bfloat16)
+    direct = run(x, None)
+    calls = []
+    forward = _kernel._forward
+    monkeypatch.setattr(_kernel, "_forward", lambda *a, **k: calls.append(k) or forward(*a, **k))
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as prof:
+        profiled = run(x, None)
+    assert any("b12x::mxfp8_linear" in event.name for event in prof.events())
+    monkeypatch.setattr(launch, "DIRECT_LAUNCH", False)
+    switched = run(x, None)
+    assert len(calls) == 2
+    assert torch.equal(profiled, direct) and torch.equal(switched, direct)

@@ -342,3 +342,40 @@ def test_the_package_imports_on_a_torch_without_cuda():
     done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True,
                           cwd=Path(__file__).resolve().parents[1])
     assert done.returncode == 0, done.stderr[-2000:]
+
+
+def test_what_keeps_a_call_on_the_custom_ops(monkeypatch):
+    """Whatever listens to operators, and the switch, which governs the GEMM's route as well."""
+    from torch.overrides import TorchFunctionMode
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from sparkinfer_b200._lib import dense_gemm, launch
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    seen = []
+
+    def ask(x):
+        seen.append(launch.plain_eager())
+        return x
+
+    x = torch.ones(3)
+    ask(x)
+    with Dispatch():
+        ask(x)
+    torch.vmap(ask)(x)
+    torch.func.jvp(ask, (x,), (x,))
+    torch.jit.trace(ask, x, check_trace=False)
+    with torch.autograd.forward_ad.dual_level():
+        ask(x)
+    with TorchFunctionMode():
+        ask(x)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]):
+        ask(x)
+    ask(x)
+    assert seen == [True] + [False] * 7 + [True]
+    assert dense_gemm._DIRECT_LAUNCH is launch.DIRECT_LAUNCH
+    monkeypatch.setattr(launch, "DIRECT_LAUNCH", False)
+    assert not launch.plain_eager()
