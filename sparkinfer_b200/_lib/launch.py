@@ -316,11 +316,14 @@ def gemm_blockscaled(kind: int, a: torch.Tensor, sfa: torch.Tensor | None, b: to
     launch.
 
     ``ldb``: bytes between the rows of an MXFP8 / FP8 ``b`` that is wider than K (one group, no
-    forced tile).
+    forced tile, all SMs).
 
     Decode shapes (see :func:`route_to_decode_kernel`; never when a tile width is forced, always
     with ``small_m=True``) go to the weight-streaming stream-K kernel, everything else to the
     persistent tiled kernels; ``block_n=_native.BLOCK_N_PAIR`` forces the CTA-pair kernel."""
+    pitched = ldb is not None and ldb != k
+    if pitched and (groups != 1 or block_n != 0 or sm_count != 0):
+        raise ValueError("ldb goes with one group, no forced tile and all SMs")
     plain = kind == _native.KIND_FP8      # no block scales: sfa / sfb are not read
     _require_cuda("a", a)
     _require_cuda("b", b)
@@ -352,19 +355,21 @@ def gemm_blockscaled(kind: int, a: torch.Tensor, sfa: torch.Tensor | None, b: to
             None if plain else sfb.data_ptr(), c.data_ptr(), dtype_code,
             alpha.data_ptr() if alpha is not None else None,
             m, n, k, ldc if ldc is not None else n, groups)
-    if ldb is not None and ldb != k:
+    if pitched:
+        name = "b12x_b200_gemm_linear"
         rc = _call_on(index, lib.b12x_b200_gemm_linear, kind, 1 if decode else 0, *head[1:4], ldb,
                       *head[4:12], work_ptr, work_bytes, ep_ref, _status_of(index).data_ptr(),
                       stream)
     elif decode:
+        name = "b12x_b200_gemm_blockscaled_smallm_grouped"
         rc = _call_on(index, lib.b12x_b200_gemm_blockscaled_smallm_grouped, *head, work_ptr,
                       work_bytes, ep_ref, sm_count, _status_of(index).data_ptr(), stream)
     else:
+        name = "b12x_b200_gemm_blockscaled_grouped"
         rc = _call_on(index, lib.b12x_b200_gemm_blockscaled_grouped, *head, block_n, sm_count,
                       work_ptr, work_bytes, ep_ref, _status_of(index).data_ptr(), stream)
     if rc != 0:
-        _native.check(rc, "b12x_b200_gemm_blockscaled_smallm_grouped" if decode
-                      else "b12x_b200_gemm_blockscaled_grouped")
+        _native.check(rc, name)
     if _CHECK_AFTER_LAUNCH:
         _after_launch(a.device)
 

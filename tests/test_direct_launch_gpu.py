@@ -100,3 +100,16 @@ def test_the_switch_and_the_profiler_see_the_op(monkeypatch):
     switched = run(x, None)
     assert len(calls) == 2
     assert torch.equal(profiled, direct) and torch.equal(switched, direct)
+
+
+@pytest.mark.parametrize("small", [True, False])
+def test_a_refused_weight_pitch_names_its_entry_point(small):
+    from sparkinfer_b200 import _native
+    from sparkinfer_b200._lib import launch
+
+    a, b = (torch.zeros((rows, 104), dtype=torch.uint8, device=DEV) for rows in (4, 128))
+    sf = torch.full((512,), 127, dtype=torch.uint8, device=DEV)
+    out = torch.zeros((4, 128), dtype=torch.bfloat16, device=DEV)
+    with pytest.raises(_native.NativeLibraryError, match="b12x_b200_gemm_linear"):
+        launch.gemm_blockscaled(_native.KIND_MXFP8, a, sf, b, sf, out, None, 4, 128, 96, ldb=104,
+                                small_m=small)

@@ -379,3 +379,13 @@ def test_what_keeps_a_call_on_the_custom_ops(monkeypatch):
     assert dense_gemm._DIRECT_LAUNCH is launch.DIRECT_LAUNCH
     monkeypatch.setattr(launch, "DIRECT_LAUNCH", False)
     assert not launch.plain_eager()
+
+
+@pytest.mark.parametrize("refused", [{"groups": 2}, {"block_n": 128}, {"sm_count": 16}])
+def test_a_weight_pitch_refuses_what_its_entry_point_cannot_take(refused):
+    from sparkinfer_b200 import _native
+    from sparkinfer_b200._lib import launch
+
+    t = torch.zeros(1, dtype=torch.uint8)
+    with pytest.raises(ValueError, match="ldb"):
+        launch.gemm_blockscaled(_native.KIND_MXFP8, t, t, t, t, t, None, 4, 128, 96, ldb=128, **refused)
