@@ -172,7 +172,10 @@ PairTailPlan plan_pair_tail(int kind, int64_t m, int64_t n, int64_t k, int64_t g
 // pair kernel was 8 % (MXFP8, FP8) and 12 % (NVFP4) off. Examples, before -> now in us: MXFP8
 // 84 x 35840 x 512 13.4 -> 8.9, 3353 x 1280 x 1024 10.9 -> 8.7, NVFP4 300 x 18432 x 1024 13.1 -> 9.2,
 // 81 x 37760 x 3584 21.0 -> 18.1.
-int choose_tile(int kind, int64_t m, int64_t n, int64_t k, int64_t groups, int sms) {
+// `scratch_bytes`: what the caller brought. Where that does not hold the partials of the split, the
+// leftover pair tiles take a round of their own.
+int choose_tile(int kind, int64_t m, int64_t n, int64_t k, int64_t groups, int sms,
+                int64_t scratch_bytes) {
   struct Cost { int block_n; int step[3], round[3], fixed; };   // MXFP8, FP4, unscaled FP8
   static const Cost costs[] = {
       {64, {27, 29, 26}, {50, 43, 30}, 370},
@@ -194,9 +197,10 @@ int choose_tile(int kind, int64_t m, int64_t n, int64_t k, int64_t groups, int s
       const int64_t tiles = ((m + 255) / 256) * ((n + 255) / 256) * groups;
       const int64_t pairs = tiles < sms / 2 ? tiles : sms / 2;
       const PairTailPlan tail = plan_pair_tail(kind, m, n, k, groups, sms);
-      const int64_t whole = tail.segments >= 2 ? tiles / pairs : (tiles + pairs - 1) / pairs;
+      const bool split = tail.segments >= 2 && scratch_bytes >= int64_t(tail.bytes);
+      const int64_t whole = split ? tiles / pairs : (tiles + pairs - 1) / pairs;
       cost = whole * (k_tiles * c.step[row] + c.round[row]) + c.fixed;
-      if (tail.segments >= 2) cost += k_tiles * c.step[row] / tail.segments + c.round[row] + kTail;
+      if (split) cost += k_tiles * c.step[row] / tail.segments + c.round[row] + kTail;
     } else {
       const int64_t tiles = ((m + 127) / 128) * ((n + c.block_n - 1) / c.block_n) * groups;
       cost = (tiles + sms - 1) / sms * (k_tiles * c.step[row] + c.round[row]) + c.fixed;
@@ -279,7 +283,8 @@ int gemm_blockscaled_impl(int kind, const void* a, const void* sfa, const void* 
   const int sms = (sm_count > 0 && sm_count < info.sm_count) ? sm_count : info.sm_count;
   if (block_n == B12X_B200_BLOCK_N_PAIR && sms < 2)
     return fail(B12X_B200_ERR_UNSUPPORTED, "the CTA-pair kernel needs two SMs");
-  const int bn = block_n != 0 ? block_n : choose_tile(kind, m, n, k, groups, sms);
+  const int64_t scratch_bytes = (workspace && aligned16(workspace)) ? workspace_bytes : 0;
+  const int bn = block_n != 0 ? block_n : choose_tile(kind, m, n, k, groups, sms, scratch_bytes);
   const bool use_pair = bn == B12X_B200_BLOCK_N_PAIR;
   const int64_t pair_tiles = ((m + 255) / 256) * ((n + 255) / 256) * groups;
 
@@ -338,8 +343,7 @@ int gemm_blockscaled_impl(int kind, const void* a, const void* sfa, const void* 
     tail.partials = nullptr;
     tail.segments = 0;
     const PairTailPlan tp = plan_pair_tail(kind, m, n, k, groups, sms);
-    if (workspace && tp.segments >= 2 && workspace_bytes >= int64_t(tp.bytes) &&
-        aligned16(workspace)) {
+    if (tp.segments >= 2 && scratch_bytes >= int64_t(tp.bytes)) {
       tail.counters = reinterpret_cast<int*>(static_cast<uint8_t*>(workspace) + kPairCounterOffset);
       tail.partials =
           reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + kWorkspaceHeaderBytes);

@@ -42,3 +42,34 @@ def test_tiles_agree(kind, m, n, k, groups):
     for block_n, c in outs.items():
         assert not torch.isnan(c).any(), block_n
         assert float((c - ref).abs().max()) <= bound, block_n
+
+
+# The plain entry point brings no scratch: 80 pair tiles on 74 pairs are then two whole rounds, and the
+# same problem runs single-CTA tiles (first shape); with 448 tiles the pair kernel runs unsplit. The
+# sums are those of the call with scratch.
+@pytest.mark.parametrize("kind,m,n,k", [
+    (_native.KIND_MXFP8, 2048, 2560, 4096), (_native.KIND_NVFP4, 2040, 2568, 7168),
+    (_native.KIND_NVFP4, 4096, 7168, 4608)])
+def test_a_call_without_scratch(kind, m, n, k):
+    import ctypes
+
+    from sparkinfer_b200._lib import launch
+
+    lib = _native.load()
+    assert lib.b12x_b200_gemm_blockscaled_workspace_bytes(kind, m, n, k, 0, 0) > 0
+    gen = torch.Generator(device=DEV).manual_seed(k)
+    a, sfa = _operand(kind, m, k, gen)
+    b, sfb = _operand(kind, n, k, gen)
+    want = torch.full((m, n), float("nan"), dtype=torch.float32, device=DEV)
+    got = want.clone()
+    launch.gemm_blockscaled(kind, a, sfa, b, sfb, want, None, m, n, k, small_m=False)
+    status = torch.zeros(4, dtype=torch.int32, device=DEV)
+    rc = lib.b12x_b200_gemm_blockscaled(
+        kind, a.data_ptr(), sfa.data_ptr(), b.data_ptr(), sfb.data_ptr(), got.data_ptr(),
+        _native.DT_FP32, None, m, n, k, n, 0, 0, status.data_ptr(),
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    _native.check(rc, "b12x_b200_gemm_blockscaled")
+    torch.cuda.synchronize()
+    launch.check_kernel_status(DEV)
+    assert int(status[0]) == 0
+    assert float((got - want).abs().max()) <= 2.0 ** -16 * float(want.abs().max())
