@@ -1,7 +1,6 @@
 """The tile an unforced GEMM gets (single-CTA widths 64 to 256, CTA pair with and without split
-leftover tiles): FP32 outputs of the unforced call and of every forced tile against the 128-column
-tile. All sum the same products in FP32, so they differ by at most 2 * K * 2^-24 of the sum of
-magnitudes, which for these operands is below sqrt(K) times the largest result."""
+leftover tiles): FP32 outputs of the unforced call and of every forced tile against an FP64 product of
+the dequantized operands."""
 
 from __future__ import annotations
 
@@ -9,7 +8,7 @@ import pytest
 import torch
 
 from sparkinfer_b200 import _native
-from test_decode_split_gpu import DEV, _operand
+from test_decode_split_gpu import DEV, _operand, assert_fp32_sums, dequantized
 
 pytestmark = pytest.mark.gpu
 
@@ -37,16 +36,44 @@ def test_tiles_agree(kind, m, n, k, groups):
                                 block_n=block_n, small_m=False)
         outs[block_n] = c
     launch.check_kernel_status(DEV)
-    ref = outs[128]
-    bound = 2.0 * k * 2.0 ** -24 * k ** 0.5 * float(ref.abs().max())
-    for block_n, c in outs.items():
-        assert not torch.isnan(c).any(), block_n
-        assert float((c - ref).abs().max()) <= bound, block_n
+    for g, ((a_g, sfa_g), (b_g, sfb_g)) in enumerate(parts):
+        if kind == _native.KIND_FP8:
+            sfa_g = sfb_g = None
+        ref = dequantized(kind, a_g, sfa_g, m, k) @ dequantized(kind, b_g, sfb_g, n, k).T
+        for c in outs.values():
+            assert_fp32_sums(c[g], ref)
+
+
+# The split of the leftover pair tiles itself, whatever tile the unforced call takes: twice the same
+# bytes (the partials are added in a fixed order), and the counters back at zero.
+@pytest.mark.parametrize("kind,m,n,k", [
+    (_native.KIND_NVFP4, 2048, 2560, 2048), (_native.KIND_MXFP8, 1536, 3328, 1024),
+    (_native.KIND_NVFP4, 2000, 2500, 1536), (_native.KIND_FP8, 1792, 2816, 1024),
+    (_native.KIND_NVFP4, 256, 19200, 1024)])
+def test_split_leftover_tiles_repeat(kind, m, n, k):
+    from sparkinfer_b200._lib import launch
+
+    need = _native.load().b12x_b200_gemm_blockscaled_workspace_bytes(
+        kind, m, n, k, _native.BLOCK_N_PAIR, 0)
+    assert need > 0
+    gen = torch.Generator(device=DEV).manual_seed(m + n)
+    a, sfa = _operand(kind, m, k, gen)
+    b, sfb = _operand(kind, n, k, gen)
+    if kind == _native.KIND_FP8:
+        sfa = sfb = None
+    outs = []
+    for _ in range(2):
+        c = torch.full((m, n), float("nan"), dtype=torch.float32, device=DEV)
+        launch.gemm_blockscaled(kind, a, sfa, b, sfb, c, None, m, n, k, block_n=_native.BLOCK_N_PAIR)
+        outs.append(c)
+    launch.check_kernel_status(DEV)
+    assert torch.equal(outs[0], outs[1])
+    assert_fp32_sums(outs[0], dequantized(kind, a, sfa, m, k) @ dequantized(kind, b, sfb, n, k).T)
+    assert int(launch.stream_workspace(need, DEV)[:65536].count_nonzero()) == 0
 
 
 # The plain entry point brings no scratch: 80 pair tiles on 74 pairs are then two whole rounds, and the
-# same problem runs single-CTA tiles (first shape); with 448 tiles the pair kernel runs unsplit. The
-# sums are those of the call with scratch.
+# same problem runs single-CTA tiles (first two shapes); with 448 tiles the pair kernel runs unsplit.
 @pytest.mark.parametrize("kind,m,n,k", [
     (_native.KIND_MXFP8, 2048, 2560, 4096), (_native.KIND_NVFP4, 2040, 2568, 7168),
     (_native.KIND_NVFP4, 4096, 7168, 4608)])
@@ -60,9 +87,7 @@ def test_a_call_without_scratch(kind, m, n, k):
     gen = torch.Generator(device=DEV).manual_seed(k)
     a, sfa = _operand(kind, m, k, gen)
     b, sfb = _operand(kind, n, k, gen)
-    want = torch.full((m, n), float("nan"), dtype=torch.float32, device=DEV)
-    got = want.clone()
-    launch.gemm_blockscaled(kind, a, sfa, b, sfb, want, None, m, n, k, small_m=False)
+    got = torch.full((m, n), float("nan"), dtype=torch.float32, device=DEV)
     status = torch.zeros(4, dtype=torch.int32, device=DEV)
     rc = lib.b12x_b200_gemm_blockscaled(
         kind, a.data_ptr(), sfa.data_ptr(), b.data_ptr(), sfb.data_ptr(), got.data_ptr(),
@@ -70,6 +95,5 @@ def test_a_call_without_scratch(kind, m, n, k):
         ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
     _native.check(rc, "b12x_b200_gemm_blockscaled")
     torch.cuda.synchronize()
-    launch.check_kernel_status(DEV)
     assert int(status[0]) == 0
-    assert float((got - want).abs().max()) <= 2.0 ** -16 * float(want.abs().max())
+    assert_fp32_sums(got, dequantized(kind, a, sfa, m, k) @ dequantized(kind, b, sfb, n, k).T)
