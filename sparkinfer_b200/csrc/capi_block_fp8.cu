@@ -14,9 +14,9 @@ namespace {
 // Weight-streaming kernel: few activation rows
 // ------------------------------------------------------------------------------------------
 // Largest M of the weight-streaming kernel. Up to 64 rows it is never behind the tiled kernel
-// (device time, weights from HBM: 64 x 54528 x 768 13.7 against 14.9 us, 64 x 7168 x 18432 29 against
-// 80). From 65 to 128 rows its activation traffic doubles, and it is ahead only where the tiled
-// kernel leaves SMs idle: 128 x 7168 x 18432 41 against 83 us, 128 x 1024 x 4608 10 against 23, but
+// (device time, weights from HBM: 64 x 54528 x 768 13.0 against 16.4 us, 64 x 7168 x 18432 31 against
+// 81). From 65 to 128 rows its activation traffic doubles, and it is ahead only where the tiled
+// kernel leaves SMs idle: 128 x 7168 x 18432 43 against 82 us, 128 x 1024 x 4608 11 against 26, but
 // 128 x 47232 x 2560 (185 tiles of 256 columns) 38 against 34.
 constexpr int64_t kBlockFp8SmallM = 128;
 constexpr int64_t kBlockFp8SmallMAlways = 64;
@@ -187,9 +187,10 @@ int launch_block_fp8_pair(const CUtensorMap& map_a, const CUtensorMap& map_b,
 
 // The CTA-pair kernel is faster per round of tiles but has more to do between two tiles. Single-CTA
 // against pair kernel in us: K = 512 100 / 109 (8192 x 16384) and 10.3 / 12.5 (1024 x 4096), K = 1536
-// 14.5 / 16.6 (700 x 5120), K = 2048 16.6 / 17.4 (200 x 14336) but 138 / 132 (8192 x 7168), K = 4096 162 / 145
-// (8192 x 4096), K = 7168 39.0 / 37.1 (256 x 7168) and 535 / 499 (4096 x 18432), K = 16384 84 / 77
-// (2048 x 2048): the line is drawn at K = 3072. An odd number of 128-row tiles costs it a row of
+// 14.5 / 16.6 (700 x 5120), K = 2048 16.6 / 17.4 (200 x 14336) but 138 / 132 (8192 x 7168), K = 3072 18.6 / 18.8
+// (160 x 2048), 20.5 / 20.6 (512 x 7168) but 60 / 58 (2048 x 7168), K = 4096 164 / 146 (8192 x 4096), K = 7168
+// 37.0 / 35.1 (256 x 7168) and 531 / 493 (4096 x 18432), K = 16384 78 / 72 (2048 x 2048): the line is drawn
+// at K = 3072, where one tile per pair is a tie and more are ahead. An odd number of 128-row tiles costs it a row of
 // tiles, so it must not need more rounds (640 x 7168: 84 pair tiles are two rounds of 74 pairs,
 // 140 single tiles are one of 148 SMs).
 bool block_fp8_pair_wins(int64_t m, int64_t n, int64_t k, int sms) {

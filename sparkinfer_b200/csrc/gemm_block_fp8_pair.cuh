@@ -28,11 +28,12 @@
 // the issuer's MMA after its wait by the fence::after_thread_sync. The arrivals therefore keep the
 // default scope: with cluster-scope release on part_empty 4096 x 18432 x 7168 takes 950 us, not 487.
 //
-// Measured (device time, single-CTA kernel -> this one): 4096 x 18432 x 7168 535 -> 499 us (2.17
-// PFLOP/s), 8192 x 4096 x 4096 162 -> 145, 512 x 4096 x 7168 39.1 -> 37.1. What is left: without the
-// promotion FMAs it runs in 414 us, without tensor-memory loads too in 388, MMAs and operand loads
-// alone take 333. Slower variants: eight promotion warps of 128 columns (557), 32-column
-// tensor-memory loads (590), register re-allocation to 104 for the promotion warps (534), packed
+// Measured (device time back to back, single-CTA kernel -> this one): 4096 x 18432 x 7168 531 -> 493 us
+// (2.20 PFLOP/s), 8192 x 4096 x 4096 164 -> 146, 256 x 7168 x 7168 37.0 -> 35.1 (one tile per pair). What is
+// left: without the promotion FMAs 4096 x 18432 x 7168 ran in 414 us, without tensor-memory loads too in
+// 388, MMAs and operand loads alone took 333, on a box where all of it took 499.
+// Slower variants: eight promotion warps of 128 columns (557), 32-column tensor-memory loads (590),
+// register re-allocation to 104 for the promotion warps (534). No faster over several runs: packed
 // FMA (492-546), three stages (496-558).
 #pragma once
 

@@ -13,8 +13,9 @@
 // (deterministic) and stores them. Partials through global memory (stream-K with a last-arriver
 // reduction) cost a fence, an atomic and loads that queue behind the ~200 KiB of weight requests
 // an SM has outstanding: 64 x 1024 x 4608 took 62 us that way, 64 x 47232 x 2560 53 us. Whole
-// tiles leave up to a tile's time of imbalance between SMs, but half of the SMs already saturate
-// HBM, so the last round runs at full bandwidth all the same.
+// tiles leave up to a tile's time of imbalance between SMs, of which the memory makes up a part: with
+// 16 x 47232 x 7168 on 37, 74, 100, 124 of the SMs the weights come at 2.2, 4.2, 5.1, 6.2 TB/s, so half of
+// the SMs still run at two thirds of the full rate.
 //
 // FP32 scales cannot ride on a block-scaled MMA, so each unit is multiplied unscaled into one of
 // four TMEM buffers (MPAD columns each) and the promotion warps add it to FP32 registers with one
@@ -26,8 +27,9 @@
 // loads queue behind the ~200 KiB of weight requests an SM has outstanding and take microseconds:
 // with the promotion warps loading their own scales 24 x 7168 x 18432 took 31 us.)
 //
-// Measured (device time, weights from HBM, before -> now): 24 x 7168 x 18432 77.6 -> 26.4 us (5.0 TB/s),
-// 1 x 1024 x 4608 21.2 -> 5.3, 64 x 47232 x 2560 32.3 -> 25.6.
+// Measured (device time back to back, weights from HBM, tiled kernel -> this one): 24 x 7168 x 18432
+// 79.5 -> 27.8 us (4.8 TB/s), 1 x 1024 x 4608 24.5 -> 6.1, 64 x 47232 x 2560 34.9 -> 26.9. Of that the wait
+// before the weight costs about 1 us, which a stream that began beside the predecessor had saved.
 //
 // Threads: warp 0 weight producer (and barrier set-up), warp 1 MMA issuer and TMEM owner, warp 2
 // activation producer, warp 3 scales, then four promotion warps per 16 or 32 activation rows, which

@@ -186,6 +186,11 @@ struct SmallMTile {
   }
 };
 
+// CTA that owns unit u when `units` are split as begin_c = c * units / ctas.
+__device__ __forceinline__ int owner_of_unit(int u, int units, int ctas) {
+  return static_cast<int>(((static_cast<long long>(u) + 1) * ctas - 1) / units);
+}
+
 // ----------------------------------------------------------------------------------------
 // Fused activation quantization: what one quantizer warp does for one unit
 // ----------------------------------------------------------------------------------------

@@ -38,9 +38,4 @@ __device__ __forceinline__ void store_rows8_packed(const P& p, uint16_t* buf, in
   }
 }
 
-// CTA that owns unit u when `units` are split as begin_c = c * units / ctas.
-__device__ __forceinline__ int owner_of_unit(int u, int units, int ctas) {
-  return static_cast<int>(((static_cast<long long>(u) + 1) * ctas - 1) / units);
-}
-
 }  // namespace b12x_b200
