@@ -21,6 +21,8 @@
 #include <cuda_fp8.h>
 #include <cstdint>
 
+#include "sm100_ptx.cuh"
+
 namespace b12x_b200 {
 
 __device__ __forceinline__ size_t sf_atom_offset(int row, int kb, int k_atoms) {
@@ -339,7 +341,9 @@ quantize_nvfp4_rows_kernel(const T* __restrict__ src, int64_t ld_src,
   quant_grid_prologue(early_release);
   QuantChunk c;
   if (!quant_chunk_of_warp(rows_cover, k_cover, c)) return;  // whole warps leave
-  const float gs = *global_scale;
+  // Not *global_scale: through a pointer to const __restrict__ that would be a load of data taken to be
+  // constant for the whole grid, free to move in front of the wait.
+  const float gs = ld_global_f32(global_scale);
   if (c.row < m && (c.chunk + 1) * kQuantChunkElems <= k)
     quantize_nvfp4_chunk<T, true>(c, src, ld_src, gs, packed, scale_mma, m, k, k_cover, k_atoms);
   else

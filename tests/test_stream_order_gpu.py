@@ -137,3 +137,43 @@ def test_decode_bias_written_just_before(n, k, dtype):
     launch.check_kernel_status(DEV)
     for i, out in enumerate(got):
         assert torch.equal(out, want[i % 2]), i
+
+
+# The global scale of the NVFP4 row quantizer, one value of the output of the GEMM launched just before.
+@pytest.mark.parametrize("m", [1, 100, 129])
+def test_global_scale_written_just_before(m):
+    from sparkinfer_b200._lib import launch
+
+    k, width = 4096, 512
+    gen = torch.Generator(device=DEV).manual_seed(m)
+    x = torch.randn((m, k), device=DEV, generator=gen).to(torch.bfloat16)
+    row, weight = (torch.full((rows, width), 0x38, dtype=torch.uint8, device=DEV) for rows in (1, 128))
+    ones = torch.ones((1, width // 128), device=DEV)
+    scale = torch.empty((1, 128), dtype=torch.float32, device=DEV)
+    alphas = [torch.tensor([v], device=DEV) for v in (1.0, 0.25)]
+    atoms = -(-m // 128) * (k // 64) * 512
+
+    def write(alpha):   # 512 products of 1.0 each
+        launch.gemm_block_fp8(row, ones, weight, ones, scale, alpha, 1, 128, width)
+
+    def quantize():
+        codes = torch.empty((m, k // 2), dtype=torch.uint8, device=DEV)
+        scales = torch.empty(atoms, dtype=torch.uint8, device=DEV)
+        launch.quantize_nvfp4_rows(x, scale[0, :1], codes, scales)
+        return codes, scales
+
+    want = []
+    for alpha in alphas:
+        write(alpha)
+        torch.cuda.synchronize()
+        want.append(quantize())
+        torch.cuda.synchronize()
+    assert float(scale[0, 0]) == 128.0 and not torch.equal(want[0][1], want[1][1])
+    got = []
+    for i in range(ROUNDS):
+        torch.cuda._sleep(2_000_000)
+        write(alphas[i % 2])
+        got.append(quantize())
+    launch.check_kernel_status(DEV)
+    for i, (codes, scales) in enumerate(got):
+        assert torch.equal(codes, want[i % 2][0]) and torch.equal(scales, want[i % 2][1]), i
